@@ -1798,13 +1798,10 @@ int dgb200_transform_sf_into_required_layout(const float* sf, int64_t stride_g, 
 }
 
 namespace {
-// The K-grouped epilogue adds its accumulators into d (TMA reductions for whole tiles, row by row for the tail of m), so d
-// must hold c before the kernel starts; the kernel then reads and writes d only.
-int prepare_k_grouped_output(CUtensorMap* tm_out, GemmParams& p, const float* c, float* d, int num_groups, int m, int n,
-                             cudaStream_t stream) {
-    if (c != d)
-        DGB_CUDA(cudaMemcpyAsync(d, c, static_cast<size_t>(num_groups) * m * n * 4, cudaMemcpyDeviceToDevice, stream));
-    p.c = d;
+// The K-grouped epilogue adds its accumulators into d where c is d (TMA reductions for whole tiles, row by row for the tail of
+// m), and reads c and writes d where they are two tensors.
+int prepare_k_grouped_output(CUtensorMap* tm_out, GemmParams& p, const float* c, float* d, int num_groups, int m, int n) {
+    p.c = c != d ? c : nullptr;
     p.tma_store = 1;  // whole 128-row tiles only: a slab must not reach into the next group's rows
     return make_tensor_map_2d(tm_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, d, static_cast<uint64_t>(n),
                               static_cast<uint64_t>(num_groups) * m, static_cast<uint64_t>(n) * 4, 16, 32, CU_TENSOR_MAP_SWIZZLE_64B);
@@ -1868,7 +1865,6 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
     }
     GemmParams p{};
     p.d = d;
-    p.c = c;
     p.d_row_stride = n;
     p.layout = ks;
     p.mode = kModeKGrouped;
@@ -1906,7 +1902,7 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
     const int grid = static_cast<int>(std::min<long long>(sms, tiles));
     // the wide tile halves the shared-memory fill per MMA cycle (the 128-wide one is bound by it)
     CUtensorMap tm_out;
-    if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n, stream))) return rc;
+    if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n))) return rc;
     if (block_n == 256) return launch_gemm<256, 4, kEpiF32Acc, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
     return launch_gemm<128, 6, kEpiF32Acc, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
 }
@@ -1930,7 +1926,6 @@ int dgb200_k_grouped_bf16_gemm_tn_contiguous(const void* a, const void* b, const
     DGB_REQUIRE(reinterpret_cast<uintptr_t>(a) % 16 == 0 && reinterpret_cast<uintptr_t>(b) % 16 == 0, "a and b must be 16-byte aligned");
     GemmParams p{};
     p.d = d;
-    p.c = c;
     p.d_row_stride = n;
     p.layout = ks;
     p.mode = kModeKGrouped;
@@ -1958,7 +1953,7 @@ int dgb200_k_grouped_bf16_gemm_tn_contiguous(const void* a, const void* b, const
     const long long tiles = static_cast<long long>(num_groups) * ((m + 127) / 128) * (n / block_n);
     const int grid = static_cast<int>(std::min<long long>(sms, tiles));
     CUtensorMap tm_out;
-    if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n, stream))) return rc;
+    if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n))) return rc;
     if (block_n == 256) return launch_gemm<256, 4, kEpiF32Acc, kKindBf16>(tm_a, tm_b, tm_a, tm_a, tm_out, p, grid, stream);
     return launch_gemm<128, 6, kEpiF32Acc, kKindBf16>(tm_a, tm_b, tm_a, tm_a, tm_out, p, grid, stream);
 }

@@ -113,7 +113,7 @@ struct GemmParams {
     const float* a_scale;
     const float* b_scales;
     const float* out_scale;
-    const float* c;  // kEpiF32Acc: unused by the kernel (the host puts c into d before the launch)
+    const float* c;  // kEpiF32Acc: d = c + accumulator, c and d two tensors; null: d already holds c (d += accumulator)
     int a_mn_major;  // BF16 kind, dense mode only: A is [k, m] with m contiguous (the reference's "tn" / "tt" forms)
     int b_mn_major;  // BF16 and FP8 x FP4 kinds: B is [groups * k, n] with n contiguous (the reference's "nn" forms; packed FP4
                      // then holds two consecutive N elements per byte) instead of [groups * n, k]
@@ -780,10 +780,28 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             if (t.group < 0) continue;
             const uint32_t as = iter % kNumAccum, aphase = (iter / kNumAccum) & 1;
             ++iter;
+            const bool warp_has_rows = static_cast<int>(q * 32) < t.rows_store;
+            // K-grouped form with c and d apart: a lane owns 16-byte chunk lane % 4 of rows lane / 4 + 8 j of the warp's
+            // 32-row x 16-column slabs. The first two slabs of c are on their way before the accumulator is waited for.
+            float4 c_next[2][4];
+            const long long c_off = kKG ? (static_cast<long long>(t.group) * p.m + t.row_start + static_cast<int>(q * 32 + lane / 4)) * p.d_row_stride +
+                                              static_cast<long long>(t.n_block) * BLOCK_N + half * kCols + (lane & 3) * 4
+                                        : 0;
+            auto load_c = [&](int slab) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (static_cast<int>(q * 32 + lane / 4) + 8 * j < t.rows_store)
+                        c_next[slab & 1][j] = __ldg(reinterpret_cast<const float4*>(p.c + c_off + 8 * j * p.d_row_stride + slab * 16));
+            };
+            if constexpr (kKG) {
+                if (p.c != nullptr) {
+                    load_c(0);
+                    load_c(1);
+                }
+            }
             ok = mbar_wait<32>(tmem_full_bar + as, aphase, abort_flag, kTimeoutTmemFull, static_cast<int>(iter));
             if (!ok) break;
             tcgen05_fence_after();
-            const bool warp_has_rows = static_cast<int>(q * 32) < t.rows_store;
             uint32_t acc[kCols];
             if (warp_has_rows) {
                 if constexpr (EPI == kEpiSwiGLU || EPI == kEpiSwiGLUNvfp4 || EPI == kEpiSwiGLUBf16) {
@@ -902,7 +920,38 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                 // D += accumulator through TMA reductions (FP32 add in the memory system; d already holds c): the warp's
                 // 32 rows x 16 columns per slab, coalesced, and no read of c through the load/store pipe. Row-per-thread
                 // loads and stores of FP32 tiles cost more than the MMAs of a tile with a short K extent.
-                if (via_tma && warp_has_rows && t.num_kb != 0) {
+                // With c in a tensor of its own the warp turns each slab through the same staging buffer, adds c (loaded two
+                // slabs ahead, 64-byte row segments) and writes d: 8 bytes per output. Copying c into d first and
+                // reducing into it moved 16 and took a pass of its own (8 groups of 4096 K rows, 4096 x 7168: 1.30 -> 1.17 ms).
+                if (p.c != nullptr) {
+                    if (warp_has_rows) {
+                        if (t.num_kb == 0) {  // empty group: d = c, the accumulator was never written
+#pragma unroll
+                            for (int i = 0; i < kCols; ++i) acc[i] = 0u;
+                        }
+#pragma unroll
+                        for (int c = 0; c < kCols / 16; ++c) {
+                            __syncwarp();
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                *stage_chunk(i) = make_uint4(acc[c * 16 + i * 4 + 0], acc[c * 16 + i * 4 + 1], acc[c * 16 + i * 4 + 2],
+                                                             acc[c * 16 + i * 4 + 3]);
+                            __syncwarp();
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const int row_in_slab = static_cast<int>(lane / 4) + 8 * j;
+                                const float4 a4 = *reinterpret_cast<const float4*>(
+                                    stage_buf + row_in_slab * 64 + (((lane & 3) ^ ((row_in_slab >> 1) & 3)) << 4));
+                                const float4 c4 = c_next[c & 1][j];
+                                if (static_cast<int>(q * 32) + row_in_slab < t.rows_store)
+                                    st_global_v4(reinterpret_cast<float*>(p.d) + c_off + 8 * j * p.d_row_stride + c * 16,
+                                                 __float_as_uint(c4.x + a4.x), __float_as_uint(c4.y + a4.y),
+                                                 __float_as_uint(c4.z + a4.z), __float_as_uint(c4.w + a4.w));
+                            }
+                            if (c + 2 < kCols / 16) load_c(c + 2);
+                        }
+                    }
+                } else if (via_tma && warp_has_rows && t.num_kb != 0) {
                     const int x0 = t.n_block * BLOCK_N + static_cast<int>(half) * kCols;
                     const int y0 = t.group * p.m + t.row_start + static_cast<int>(q) * 32;
 #pragma unroll
@@ -1003,7 +1052,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                 } else if constexpr (EPI == kEpiF32Acc) {
                     // tiles with fewer than 128 rows (the tail of m): d += accumulator row by row (d already holds c; an
                     // empty group adds nothing: its accumulator was never written)
-                    if (!via_tma && t.num_kb != 0) {
+                    if (!via_tma && t.num_kb != 0 && p.c == nullptr) {
                         const long long off = (static_cast<long long>(t.group) * p.m + row) * p.d_row_stride +
                                               static_cast<long long>(t.n_block) * BLOCK_N + half * kCols;
                         float* dst = reinterpret_cast<float*>(p.d) + off;
