@@ -27,26 +27,42 @@ bool use_pdl();  // the "pdl" tuning knob (set_pdl)
 // (reference: the launch attribute in csrc/jit/handle.hpp:77, switched by set_pdl, csrc/apis/runtime.hpp:24-28). Only
 // kernels whose first statement is pdl_prologue() may be launched this way.
 template <typename... Params, typename... Args>
-cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream, bool pdl,
-                          Args&&... args) {
+cudaError_t launch_kernel_in_clusters(int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes,
+                                      cudaStream_t stream, bool pdl, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(cluster);
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = static_cast<unsigned>(n);
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-template <int BLOCK_N, int kStages, int EPI, int kKind = kKindFp8Fp4>
+template <typename... Params, typename... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream, bool pdl,
+                          Args&&... args) {
+    return launch_kernel_in_clusters(1, kernel, grid, block, smem_bytes, stream, pdl, std::forward<Args>(args)...);
+}
+
+template <int BLOCK_N, int kStages, int EPI, int kKind = kKindFp8Fp4, bool kPair = false>
 int launch_gemm(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_sfa, const CUtensorMap& tm_sfb,
                 const CUtensorMap& tm_out, const GemmParams& p, int grid, cudaStream_t stream) {
-    using L = GemmSmem<BLOCK_N, kStages, kKind, EPI == kEpiF32Acc>;
-    auto kernel = dgb200_grouped_gemm_kernel<BLOCK_N, kStages, EPI, kKind>;
+    using L = GemmSmem<BLOCK_N, kStages, kKind, EPI == kEpiF32Acc, kPair>;
+    auto kernel = dgb200_grouped_gemm_kernel<BLOCK_N, kStages, EPI, kKind, kPair>;
     static bool configured = false;  // per instantiation; the attribute is per device function, set on every device once
     static int configured_device = -1;
     int dev = 0;
@@ -56,7 +72,8 @@ int launch_gemm(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensor
         configured = true;
         configured_device = dev;
     }
-    DGB_CUDA(launch_kernel(kernel, dim3(grid), dim3(kGemmThreads), L::kDynamicBytes, stream, use_pdl(), tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p));
+    DGB_CUDA(launch_kernel_in_clusters(kPair ? 2 : 1, kernel, dim3(grid), dim3(kGemmThreads), L::kDynamicBytes, stream, use_pdl(), tm_a, tm_b,
+                                       tm_sfa, tm_sfb, tm_out, p));
     return 0;
 }
 
@@ -79,12 +96,14 @@ struct GemmCall {
     int b_is_fp4;
     int epilogue;
     int max_tiles;  // upper bound on tiles, <= 0 if unknown
+    long long expected_rows;  // rows per group the caller expects, <= 0 if it does not say
 };
 
 // Process-wide tuning knobs (defaults are the measured best on B200).
 struct Tuning {
     int swap_ab = -1;  // layer GEMMs: tokens on the UMMA N side (-1 = by expected rows per expert, 0 = never, 1 = always)
     int block_n = 0;  // 0 = automatic
+    int pair = -1;  // GEMMs on CTA pairs: -1 = by size (use_pairs), 0 = never, 1 = wherever the form exists
     int mlp_kernel = -1;  // FP8 x FP4 layer GEMMs: 0 = separate gate/up and down kernels (tokens-on-M / swapped split),
                           // 1 = the fused expert-MLP kernel on single CTAs, 2 = on CTA pairs; -1 = not yet read from
                           // the environment (DGB200_MLP_KERNEL, default below)
@@ -116,6 +135,30 @@ int mlp_kernel_choice() {
         if (t.mlp_kernel < 0 || t.mlp_kernel > 2) t.mlp_kernel = kDefaultMlpKernel;
     }
     return t.mlp_kernel;
+}
+
+// Pipeline stages of the pair kernels (the operand stages are 32 KB; NVFP4 adds 6 KB of scale factors to each, the others 1.5)
+constexpr int kPairStages = 6, kPairStagesNvfp4 = 5;
+
+bool use_pairs(const GemmCall& c, int block_n, int sms) {
+    const GemmParams& p = c.p;
+    if (tuning().pair == 0 || block_n != 256 || sms < 2) return false;
+    if (p.mode != kModeDense && p.mode != kModePsum && p.mode != kModeMasked) return false;
+    if (p.rows_lo != 0 || p.rows_hi != 0 || p.ret_src != nullptr || p.push != nullptr) return false;
+    if (p.row_part == kRowsTail) return false;
+    if (tuning().pair == 1 || p.row_part == kRowsPairs) return true;
+    if (p.mode == kModeDense) {
+        // A pair tile takes about 0.87 of the time two single-CTA tiles take on the same two SMs (FP8 8192^3: 0.80, 4000 x
+        // 7168 x 2048: 0.85, BF16 4096 x 7168 x 2048: 0.90); with twice the granularity it may need another wave.
+        const long long nb = p.n / 256;
+        const long long single = (p.m + 127ll) / 128 * nb, pairs = (p.m + 255ll) / 256 * nb;
+        const long long waves1 = (single + sms - 1) / sms, waves2 = (pairs + sms / 2 - 1) / (sms / 2);
+        return p.m > 128 && waves2 * 87 < waves1 * 100;
+    }
+    // Grouped: half a pair tile is lost on every second group. From 512 rows per group on that is less than what the pairs
+    // gain (8 groups of 1024 to 2048 rows, N 4096, K 7168: NVFP4 0.86 of the single-CTA time, BF16 0.95, FP8 x FP4 0.97). The
+    // psum layout only tells the rows the buffer holds, of which some are padding or free.
+    return c.expected_rows >= (p.mode == kModePsum ? 768 : 512);
 }
 
 int run_gemm(GemmCall& c, cudaStream_t stream) {
@@ -175,6 +218,10 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     DGB_REQUIRE(!swiglu || p.n % 256 == 0, "the gate/up GEMM needs n (%d) to be a multiple of 256", p.n);
     const int block_n = swiglu ? 256 : (tuning().block_n != 0 ? tuning().block_n : (p.n % 256 == 0 ? 256 : 128));
     DGB_REQUIRE((block_n == 128 || block_n == 256) && p.n % block_n == 0, "block_n %d does not divide n %d", block_n, p.n);
+    int sms = 0;
+    rc = effective_num_sms(&sms);
+    if (rc) return rc;
+    const bool pair = use_pairs(c, block_n, sms);
     if (!bf16) {
         rc = make_tensor_map_2d(&tm_sfb, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfb, static_cast<uint64_t>(c.sfb_k_stride),
                                 static_cast<uint64_t>(packed_k_b) * p.num_groups, static_cast<uint64_t>(c.sfb_k_stride) * 4,
@@ -199,7 +246,7 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     if (rc) return rc;
     if (bf16) tm_sfa = tm_sfb = tm_a;  // valid maps for the kernel's descriptor prefetch; never used for a copy
     const uint64_t b_rows = static_cast<uint64_t>(p.num_groups) * p.n;
-    const uint32_t BLOCK_N = static_cast<uint32_t>(block_n);
+    const uint32_t BLOCK_N = static_cast<uint32_t>(pair ? block_n / 2 : block_n);  // channels of B that one CTA loads
     if (bf16) {
         if (c.b_mn_major)
             rc = make_tensor_map_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, c.b, static_cast<uint64_t>(p.n),
@@ -249,7 +296,7 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     p.tma_store = 0;
     // NVFP4: only the BF16 epilogue (the down GEMM: few K blocks per tile, so its store burst weighs most) trades a
     // pipeline stage for the staging buffers.
-    const bool nvfp4_staged = nvfp4 && block_n == 256 && c.epilogue == kEpiBF16;
+    const bool nvfp4_staged = nvfp4 && block_n == 256 && c.epilogue == kEpiBF16;  // (the pair form stages either way)
     if (block_n == 256 && c.epilogue == kEpiSwiGLUBf16) {
         rc = make_tensor_map_2d(&tm_out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, p.act_q, static_cast<uint64_t>(p.n / 2),
                                 static_cast<uint64_t>(c.a_rows_total), static_cast<uint64_t>(p.act_q_row_stride), 32, 32,
@@ -270,10 +317,26 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
         p.tma_store = c.whole_tile_stores ? 2 : 1;
     }
 
-    int sms = 0;
-    rc = effective_num_sms(&sms);
-    if (rc) return rc;
     int grid = sms;
+    if (pair) {
+        // (the number of 256 x 256 tiles is at most half the number of 128 x 256 ones, rounded up per group)
+        grid = sms / 2 * 2;
+        if (c.max_tiles > 0) grid = std::min(grid, std::max(2, (c.max_tiles + 1) / 2 * 2));
+        switch (c.epilogue) {
+            case kEpiBF16:
+                if (bf16) return launch_gemm<256, kPairStages, kEpiBF16, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+                if (nvfp4) return launch_gemm<256, kPairStagesNvfp4, kEpiBF16, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+                return launch_gemm<256, kPairStages, kEpiBF16, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            case kEpiF32:
+                if (bf16) return launch_gemm<256, kPairStages, kEpiF32, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+                if (nvfp4) return launch_gemm<256, kPairStagesNvfp4, kEpiF32, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+                return launch_gemm<256, kPairStages, kEpiF32, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            case kEpiSwiGLU: return launch_gemm<256, kPairStages, kEpiSwiGLU, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            case kEpiSwiGLUBf16: return launch_gemm<256, kPairStages, kEpiSwiGLUBf16, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            case kEpiSwiGLUNvfp4: return launch_gemm<256, kPairStagesNvfp4, kEpiSwiGLUNvfp4, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            default: return fail(DGB200_EINVAL, "unknown epilogue %d", c.epilogue);
+        }
+    }
     if (c.max_tiles > 0) grid = std::min(grid, c.max_tiles);
 
     if (c.max_tiles > 0 && block_n == 256) grid = std::min(grid, std::max(1, c.max_tiles / 2));
@@ -771,10 +834,39 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
     }
     const LayerOrientation orient = layer_orientation(quant.kind, E, hidden, intermediate_hidden, expected_rows_per_expert);
     int rc = 0;
+    // Groups of many rows: CTA pairs for whole 256-row tiles, the single-CTA kernel for what is left of each group (at most
+    // 128 rows) on the side stream. Whole layers under sustained load, single-CTA -> pairs and tails (all rows through
+    // pairs): FP8 x MXFP4, 64 experts: 256 rows each 1.00 -> 0.91 ms (0.95), 375 rows 1.33 -> 1.20 (1.28), 1024 rows 3.28 ->
+    // 2.79 (2.83). NVFP4, 256 experts of 512 rows: 4.76 -> 4.29 ms (4.35); of 250 rows no difference. BF16: 512 rows 3.46 -> 3.24
+    // (3.32); 375 rows 1.33 -> 1.37.
+    const long long pair_rows = nvfp4 ? 384 : (bf16 ? 448 : 192);
+    const bool pairs_and_tails = orient == kOrientM && (tuning().pair == 1 || (tuning().pair == -1 && expected_rows_per_expert >= pair_rows)) &&
+                                 E <= kMaxCachedGroups && ret == nullptr && push == nullptr && (2 * intermediate_hidden) % 256 == 0 && hidden % 256 == 0 &&
+                                 (tuning().block_n == 0 || tuning().block_n == 256);
+    // `first` on the caller's stream and `second` on the side stream, concurrently
+    auto run_both = [&](GemmCall& first, auto&& second) -> int {
+        SideStream* side = nullptr;
+        int rc1 = side_stream_for_current_device(&side);
+        if (rc1) return rc1;
+        std::lock_guard<std::mutex> lock(side->mu);
+        DGB_CUDA(cudaEventRecord(side->fork, stream));
+        DGB_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
+        rc1 = run_gemm(first, stream);
+        if (rc1 == 0) rc1 = second(side->stream);
+        // join even after a failed launch, so that the side stream never runs ahead of the caller's stream
+        DGB_CUDA(cudaEventRecord(side->join, side->stream));
+        DGB_CUDA(cudaStreamWaitEvent(stream, side->join, 0));
+        return rc1;
+    };
     auto run_split = [&](GemmCall& c) -> int {
-        if (orient == kOrientM) return run_gemm(c, stream);
         if (orient == kOrientSwapAll) return run_gemm_swap(c, stream);
+        if (orient == kOrientM && !pairs_and_tails) return run_gemm(c, stream);
         GemmCall c2 = c;
+        if (orient == kOrientM) {
+            c.p.row_part = kRowsPairs;
+            c2.p.row_part = kRowsTail;
+            return run_both(c, [&](cudaStream_t side) { return run_gemm(c2, side); });
+        }
         const int split_lo = tuning().swap_ab == 2 ? 1 : 129;  // 2: every expert that fits one token tile (experiments)
         c.p.rows_lo = c2.p.rows_lo = split_lo;
         c.p.rows_hi = c2.p.rows_hi = kSwapMaxTok;
@@ -786,26 +878,16 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
             c2.p.d = base + l.l1_tmp;
             c2.p.d_row_stride = 2 * intermediate_hidden;
         }
-        SideStream* side = nullptr;
-        int rc1 = side_stream_for_current_device(&side);
-        if (rc1) return rc1;
-        std::lock_guard<std::mutex> lock(side->mu);
-        DGB_CUDA(cudaEventRecord(side->fork, stream));
-        DGB_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
-        rc1 = run_gemm(c, stream);
-        if (rc1 == 0) rc1 = run_gemm_swap(c2, side->stream);
-        if (rc1 == 0 && gate_up) {
+        return run_both(c, [&](cudaStream_t side) -> int {
+            const int rc1 = run_gemm_swap(c2, side);
+            if (rc1 || !gate_up) return rc1;
             const dim3 grid((kSwapMaxTok + 7) / 8, num_call_experts);
-            dgb200_swiglu_requant_rows_kernel<<<grid, 256, 0, side->stream>>>(
+            dgb200_swiglu_requant_rows_kernel<<<grid, 256, 0, side>>>(
                 reinterpret_cast<const __nv_bfloat16*>(base + l.l1_tmp), reinterpret_cast<const int*>(base + l.expert_start), expert_end,
                 split_lo, kSwapMaxTok, intermediate_hidden, c.p.row_weight, c.p.clamp, c.p.fast_math, c.p.act_q, c.p.act_q_row_stride,
                 reinterpret_cast<unsigned*>(c.p.act_sf), c.p.act_sf_k_stride, first_expert);
-            if (cudaGetLastError() != cudaSuccess) rc1 = fail(DGB200_ECUDA, "launch of the SwiGLU finisher failed");
-        }
-        // join even after a failed launch, so that the side stream never runs ahead of the caller's stream
-        DGB_CUDA(cudaEventRecord(side->join, side->stream));
-        DGB_CUDA(cudaStreamWaitEvent(stream, side->join, 0));
-        return rc1;
+            return cudaGetLastError() != cudaSuccess ? fail(DGB200_ECUDA, "launch of the SwiGLU finisher failed") : 0;
+        });
     };
     {
         GemmCall c{};
@@ -1478,6 +1560,9 @@ int dgb200_set_tuning(const char* name, int32_t value) {
     } else if (std::strcmp(name, "block_n") == 0) {
         DGB_REQUIRE(value == 0 || value == 128 || value == 256, "block_n must be 0 (automatic), 128 or 256");
         tuning().block_n = value;
+    } else if (std::strcmp(name, "pair") == 0) {
+        DGB_REQUIRE(value >= -1 && value <= 1, "pair must be -1 (automatic), 0 (never) or 1 (wherever the form exists)");
+        tuning().pair = value;
     } else if (std::strcmp(name, "fused_dispatch") == 0) {
         DGB_REQUIRE(value >= 0 && value <= kMaxEpPhases, "fused_dispatch must be 0 (off), 1 (on, %d phases) or a phase count up to %d", kMaxEpPhases, kMaxEpPhases);
         tuning().fused_dispatch = value;
@@ -1568,6 +1653,7 @@ int run_m_grouped_contiguous(
     p.store_padding = store_padding;
     const long long m_blocks = (static_cast<long long>(m) + 127) / 128 + (p.mode == kModePsum ? num_groups : 0);
     c.max_tiles = static_cast<int>(std::min<long long>(m_blocks * (n / 128 > 0 ? n / 128 : 1), 1 << 30));
+    c.expected_rows = num_groups > 0 ? m / num_groups : 0;
     return run_gemm(c, static_cast<cudaStream_t>(stream));
 }
 }  // namespace
@@ -1641,7 +1727,6 @@ int dgb200_m_grouped_fp8_fp4_gemm_nt_masked(
     void* d, int64_t d_row_stride, const int32_t* masked_m,
     int32_t num_groups, int32_t max_m, int32_t n, int32_t k, int32_t expected_m,
     int32_t gran_k_a, int32_t gran_k_b, int32_t b_is_fp4, int32_t d_is_fp32, void* stream) {
-    (void)expected_m;
     DGB_REQUIRE(max_m > 0 && max_m % 4 == 0, "max_m (%d) must be a positive multiple of 4", max_m);
     DGB_REQUIRE(d != nullptr, "null output");
     DGB_REQUIRE(d_row_stride >= n && (d_row_stride * (d_is_fp32 ? 4 : 2)) % 16 == 0,
@@ -1674,6 +1759,7 @@ int dgb200_m_grouped_fp8_fp4_gemm_nt_masked(
     p.gran_b = gran_k_b;
     p.store_padding = 0;
     c.max_tiles = 0;
+    c.expected_rows = std::min(expected_m, max_m);
     return run_gemm(c, static_cast<cudaStream_t>(stream));
 }
 
@@ -1681,7 +1767,7 @@ namespace {
 // Shared body of the BF16 GEMM entry points: A [rows, k] and B [num_groups * n, k] BF16 K-major, D BF16 or FP32.
 int run_bf16_gemm(const void* a, int64_t a_row_stride, int32_t a_mn_major, const void* b, int64_t b_row_stride, int32_t b_mn_major, void* d,
                   int64_t d_row_stride, int32_t d_is_fp32, int32_t accumulate, const int32_t* layout, int mode, long long a_rows_total, int32_t m, int32_t n, int32_t k,
-                  int32_t num_groups, int32_t alignment, int32_t store_padding, int max_tiles, void* stream) {
+                  int32_t num_groups, int32_t alignment, int32_t store_padding, int max_tiles, long long expected_rows, void* stream) {
     DGB_REQUIRE(d != nullptr || a_rows_total == 0, "null output");
     DGB_REQUIRE(d_row_stride >= n && (d_row_stride * (d_is_fp32 ? 4 : 2)) % 16 == 0,
                 "d row stride must cover n and keep rows 16-byte aligned");
@@ -1712,6 +1798,7 @@ int run_bf16_gemm(const void* a, int64_t a_row_stride, int32_t a_mn_major, const
     p.accumulate = accumulate ? 1 : 0;
     DGB_REQUIRE(!accumulate || d_is_fp32, "accumulation needs a float32 d");
     c.max_tiles = max_tiles;
+    c.expected_rows = expected_rows;
     return run_gemm(c, static_cast<cudaStream_t>(stream));
 }
 }  // namespace
@@ -1730,16 +1817,16 @@ int dgb200_m_grouped_bf16_gemm_nt_contiguous(const void* a, int64_t a_row_stride
     const long long m_blocks = (static_cast<long long>(m) + 127) / 128 + (mode == kModePsum ? num_groups : 0);
     const int max_tiles = static_cast<int>(std::min<long long>(m_blocks * (n / 128 > 0 ? n / 128 : 1), 1 << 30));
     return run_bf16_gemm(a, a_row_stride, 0, b, b_row_stride, b_mn_major, d, d_row_stride, d_is_fp32, 0, grouped_layout, mode, m, m, n, k,
-                         num_groups, alignment, store_padding, max_tiles, stream);
+                         num_groups, alignment, store_padding, max_tiles, num_groups > 0 ? m / num_groups : 0, stream);
 }
 
 int dgb200_m_grouped_bf16_gemm_nt_masked(const void* a, const void* b, void* d, int64_t d_row_stride, const int32_t* masked_m,
                                          int32_t num_groups, int32_t max_m, int32_t n, int32_t k, int32_t expected_m,
                                          int32_t d_is_fp32, void* stream) {
-    (void)expected_m;
     DGB_REQUIRE(max_m > 0 && max_m % 4 == 0, "max_m (%d) must be a positive multiple of 4", max_m);
     return run_bf16_gemm(a, k, 0, b, k, 0, d, d_row_stride, d_is_fp32, 0, masked_m, kModeMasked,
-                         static_cast<long long>(num_groups) * max_m, max_m, n, k, num_groups, 4, 0, 0, stream);
+                         static_cast<long long>(num_groups) * max_m, max_m, n, k, num_groups, 4, 0, 0,
+                         std::min(expected_m, max_m), stream);
 }
 
 int dgb200_bf16_gemm_nt(const void* a, int64_t a_row_stride, int32_t a_mn_major, const void* b, int64_t b_row_stride,
@@ -1751,7 +1838,7 @@ int dgb200_bf16_gemm_nt(const void* a, int64_t a_row_stride, int32_t a_mn_major,
     DGB_REQUIRE(!a_mn_major || m % 8 == 0, "an MN-major a needs m (%d) to be a multiple of 8", m);
     return run_bf16_gemm(a, a_row_stride, a_mn_major, b, b_row_stride, b_mn_major, d, d_row_stride, d_is_fp32, accumulate, nullptr,
                          kModeDense, m, m, n, k, 1, 128,
-                         0, max_tiles, stream);
+                         0, max_tiles, 0, stream);
 }
 
 int dgb200_per_token_cast_to_fp8(const void* x, int64_t x_row_stride, int32_t rows, int32_t k, int32_t gran_k, void* q,
@@ -1798,6 +1885,17 @@ int dgb200_transform_sf_into_required_layout(const float* sf, int64_t stride_g, 
 }
 
 namespace {
+bool use_pairs_k_grouped(int m, int block_n, int sms) {
+    if (tuning().pair == 0 || block_n != 256 || sms < 2) return false;
+    return m > 128 || tuning().pair == 1;
+}
+
+int k_grouped_grid(bool pair, int num_groups, int m, int n, int block_n, int sms) {
+    const int tile_m = pair ? 256 : 128, ctas = pair ? 2 : 1;
+    const long long tiles = static_cast<long long>(num_groups) * ((m + tile_m - 1) / tile_m) * (n / block_n);
+    return static_cast<int>(std::min<long long>(sms / ctas, tiles)) * ctas;
+}
+
 // The K-grouped epilogue adds its accumulators into d where c is d (TMA reductions for whole tiles, row by row for the tail of
 // m), and reads c and writes d where they are two tensors.
 int prepare_k_grouped_output(CUtensorMap* tm_out, GemmParams& p, const float* c, float* d, int num_groups, int m, int n) {
@@ -1880,9 +1978,13 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
     // 1.7 - 2.0 PFLOP/s over 1024 .. 8192 K rows per group).
     const int block_n = tuning().block_n != 0 ? tuning().block_n : (n % 256 == 0 ? 256 : 128);
     DGB_REQUIRE(n % block_n == 0, "block_n %d does not divide n %d", block_n, n);
-    p.b_tx_bytes = block_n * 128;
+    int sms = 0;
+    int rc = effective_num_sms(&sms);
+    if (rc) return rc;
+    const bool pair = use_pairs_k_grouped(m, block_n, sms);
+    p.b_tx_bytes = (pair ? block_n / 2 : block_n) * 128;
     CUtensorMap tm_a, tm_b, tm_sfa, tm_sfb;
-    int rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),
+    rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),
                                 static_cast<uint64_t>(m), 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     rc = make_tensor_map_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, b, static_cast<uint64_t>(n), static_cast<uint64_t>(sum_k),
@@ -1895,14 +1997,10 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
                             static_cast<uint64_t>(kp_rows), static_cast<uint64_t>(aligned_n) * 4, static_cast<uint32_t>(block_n), 1,
                             CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    int sms = 0;
-    rc = effective_num_sms(&sms);
-    if (rc) return rc;
-    const long long tiles = static_cast<long long>(num_groups) * ((m + 127) / 128) * (n / block_n);
-    const int grid = static_cast<int>(std::min<long long>(sms, tiles));
-    // the wide tile halves the shared-memory fill per MMA cycle (the 128-wide one is bound by it)
+    const int grid = k_grouped_grid(pair, num_groups, m, n, block_n, sms);
     CUtensorMap tm_out;
     if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n))) return rc;
+    if (pair) return launch_gemm<256, kPairStages, kEpiF32Acc, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
     if (block_n == 256) return launch_gemm<256, 4, kEpiF32Acc, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
     return launch_gemm<128, 6, kEpiF32Acc, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
 }
@@ -1939,21 +2037,22 @@ int dgb200_k_grouped_bf16_gemm_tn_contiguous(const void* a, const void* b, const
     p.sf_transposed = 1;
     const int block_n = tuning().block_n != 0 ? tuning().block_n : (n % 256 == 0 ? 256 : 128);
     DGB_REQUIRE(n % block_n == 0, "block_n %d does not divide n %d", block_n, n);
-    p.b_tx_bytes = block_n * 128;
+    int sms = 0;
+    int rc = effective_num_sms(&sms);
+    if (rc) return rc;
+    const bool pair = use_pairs_k_grouped(m, block_n, sms);
+    p.b_tx_bytes = (pair ? block_n / 2 : block_n) * 128;
     CUtensorMap tm_a, tm_b;
-    int rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),
+    rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),
                                 static_cast<uint64_t>(m) * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     rc = make_tensor_map_2d(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, static_cast<uint64_t>(n), static_cast<uint64_t>(sum_k),
                             static_cast<uint64_t>(n) * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    int sms = 0;
-    rc = effective_num_sms(&sms);
-    if (rc) return rc;
-    const long long tiles = static_cast<long long>(num_groups) * ((m + 127) / 128) * (n / block_n);
-    const int grid = static_cast<int>(std::min<long long>(sms, tiles));
+    const int grid = k_grouped_grid(pair, num_groups, m, n, block_n, sms);
     CUtensorMap tm_out;
     if ((rc = prepare_k_grouped_output(&tm_out, p, c, d, num_groups, m, n))) return rc;
+    if (pair) return launch_gemm<256, kPairStages, kEpiF32Acc, kKindBf16, true>(tm_a, tm_b, tm_a, tm_a, tm_out, p, grid, stream);
     if (block_n == 256) return launch_gemm<256, 4, kEpiF32Acc, kKindBf16>(tm_a, tm_b, tm_a, tm_a, tm_out, p, grid, stream);
     return launch_gemm<128, 6, kEpiF32Acc, kKindBf16>(tm_a, tm_b, tm_a, tm_a, tm_out, p, grid, stream);
 }
@@ -2328,6 +2427,7 @@ int dgb200_m_grouped_nvfp4_gemm_nt_contiguous(
     p.a_scale = a_scale;
     p.b_scales = b_scales;
     c.max_tiles = 0;
+    c.expected_rows = num_groups > 0 ? m / num_groups : 0;
     return run_gemm(c, static_cast<cudaStream_t>(stream));
 }
 

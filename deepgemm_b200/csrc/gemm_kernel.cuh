@@ -78,6 +78,12 @@ struct PushWork {
     unsigned long long acts_base[kMaxRanks], sf_base[kMaxRanks], weight_base[kMaxRanks], src_base[kMaxRanks];  // per rank
 };
 
+enum RowPart : int {
+    kRowsAll = 0,
+    kRowsPairs = 1,  // what 256-row tiles hold: all but a last remainder of at most 128 rows
+    kRowsTail = 2,   // that remainder
+};
+
 struct GemmParams {
     // Scale factors are read through tensor maps over int32 [groups * packed_k, aligned MN] (packed UE8M0, MN-major):
     // int (group, kp, row) sits at outer coordinate group * packed_k + kp, inner coordinate row.
@@ -96,6 +102,9 @@ struct GemmParams {
                              // with different tile orientations split the groups of one GEMM by size.
     int group_begin, group_end;  // psum / masked layouts: only groups in [group_begin, group_end) are computed; {0, 0} = all.
                                  // The expert-parallel layer runs its experts phase by phase.
+    // psum layouts without store_padding: which rows of a group are computed (RowPart). Lets the pair kernel and the single-CTA
+    // kernel share one GEMM: a 256-row pair tile with 128 rows or fewer to compute would do twice the work it has.
+    int row_part;
     // SwiGLU epilogue only
     unsigned char* act_q;        // e4m3 [rows, n/2]
     int tma_store;               // epilogue stores through shared memory + TMA (BLOCK_N = 256, FP8 x FP4 kind): 0 never,
@@ -183,16 +192,22 @@ __device__ __forceinline__ bool group_selected(const GemmParams& p, int rows) {
     return p.rows_skip ? !inside : inside;
 }
 
-template <int BLOCK_N, bool kKGrouped = false>
+// kPair: a tile is 256 rows tall and belongs to a cluster of two CTAs, each of which sees its own 128 rows (rows_store may
+// then be zero or negative for the second one, which still takes part in the tile's MMAs).
+template <int BLOCK_N, bool kKGrouped = false, bool kPair = false>
 struct TileScheduler {
+    static constexpr int kTileM = kPair ? 256 : 128;
     const GemmParams& p;
     const GroupTable tab;
     int num_n_blocks;
-    int tile;  // next global tile index of this CTA
+    int tile;    // next global tile index of this CTA (or pair)
+    int stride;  // CTAs (or pairs) of the grid
+    int sub;     // first row of this CTA inside the tile
     int g, tiles_before_g;
 
     __device__ TileScheduler(const GemmParams& params, const GroupTable& table)
-        : p(params), tab(table), num_n_blocks(params.n / BLOCK_N), tile(static_cast<int>(blockIdx.x)), g(0),
+        : p(params), tab(table), num_n_blocks(params.n / BLOCK_N), tile(static_cast<int>(blockIdx.x) / (kPair ? 2 : 1)),
+          stride(static_cast<int>(gridDim.x) / (kPair ? 2 : 1)), sub(kPair ? static_cast<int>(blockIdx.x & 1) * 128 : 0), g(0),
           tiles_before_g(0) {}
 
     // First row, valid rows and rows to store of one group, from the layout words.
@@ -207,6 +222,17 @@ struct TileScheduler {
             start = (prev_end + p.alignment - 1) / p.alignment * p.alignment;
             const int end = lay[group];
             rows = max(end - start, 0);
+            if (p.row_part != kRowsAll) {
+                const int rest = rows % 256, tail = rest <= 128 ? rest : 0;
+                if (p.row_part == kRowsTail) {
+                    start += rows - tail;
+                    rows = tail;
+                } else {
+                    rows -= tail;
+                }
+                rows_store = rows;
+                return;
+            }
             const int aligned_end = min((end + p.alignment - 1) / p.alignment * p.alignment, p.m);
             rows_store = p.store_padding ? max(aligned_end - start, 0) : rows;
         }
@@ -216,11 +242,11 @@ struct TileScheduler {
         int mb = 0;
         while (local >= num_n_blocks) { local -= num_n_blocks; ++mb; }  // groups are a few M blocks tall
         t.n_block = local;
-        t.row_start = start + mb * 128;
-        t.sf_row_start = p.mode == kModeMasked ? mb * 128 : t.row_start;
-        t.rows_store = min(128, rows_store - mb * 128);
+        t.row_start = start + mb * kTileM + sub;
+        t.sf_row_start = p.mode == kModeMasked ? mb * kTileM + sub : t.row_start;
+        t.rows_store = min(128, rows_store - mb * kTileM - sub);
         t.group = group;
-        tile += static_cast<int>(gridDim.x);
+        tile += stride;
     }
 
     // Returns false when this CTA has no more tiles. A tile with group < 0 must be skipped by every role.
@@ -228,30 +254,31 @@ struct TileScheduler {
         if constexpr (kKGrouped) {
             // every group has the same (m blocks x n blocks) output tiles; the table holds (K blocks, first K row,
             // first packed scale row) per group
-            const int per_group = (p.m + 127) / 128 * num_n_blocks;
+            const int per_group = (p.m + kTileM - 1) / kTileM * num_n_blocks;
             if (tile >= p.num_groups * per_group) return false;
             const int group = tile / per_group;
             const int local = tile - group * per_group;
             const int mb = local / num_n_blocks;
             t.n_block = local - mb * num_n_blocks;
-            t.row_start = t.sf_row_start = mb * 128;
-            t.rows_store = min(128, p.m - mb * 128);
+            t.row_start = t.sf_row_start = mb * kTileM + sub;
+            t.rows_store = min(128, p.m - t.row_start);
             t.group = group;
             t.num_kb = tab.lay[group];
             t.k_row_start = tab.start[group];
             t.sf_kp0 = tab.tiles_end[group];
-            tile += static_cast<int>(gridDim.x);
+            tile += stride;
             return true;
         }
         if (p.mode == kModeRowIds || p.mode == kModeDense) {
-            const int num_m_blocks = (p.m + 127) / 128;
+            const int num_m_blocks = (p.m + kTileM - 1) / kTileM;
             if (tile >= num_m_blocks * num_n_blocks) return false;
             const int mb = tile / num_n_blocks;
             t.n_block = tile - mb * num_n_blocks;
-            t.row_start = t.sf_row_start = mb * 128;
+            t.row_start = t.sf_row_start = mb * kTileM + sub;
             t.rows_store = min(128, p.m - t.row_start);
+            // (pairs serve no row-id layouts: the two halves of their tiles could belong to different groups)
             t.group = p.mode == kModeDense ? 0 : __ldg(p.layout + t.row_start);
-            tile += static_cast<int>(gridDim.x);
+            tile += stride;
             return true;
         }
         if (tab.cached) {
@@ -272,7 +299,7 @@ struct TileScheduler {
         while (g < p.num_groups) {
             int start, rows, rows_store;
             group_extent(p, tab.lay, g, start, rows, rows_store);
-            const int tiles_g = (group_selected(p, rows) && group_in_range(p, g)) ? (max(rows, rows_store) + 127) / 128 * num_n_blocks : 0;
+            const int tiles_g = (group_selected(p, rows) && group_in_range(p, g)) ? (max(rows, rows_store) + kTileM - 1) / kTileM * num_n_blocks : 0;
             if (tile < tiles_before_g + tiles_g) {
                 fill(t, g, start, rows_store, tile - tiles_before_g);
                 return true;
@@ -284,11 +311,11 @@ struct TileScheduler {
     }
 };
 
-template <int BLOCK_N, int kStages, int kKind = kKindFp8Fp4, bool kAlwaysStaged = false>
+template <int BLOCK_N, int kStages, int kKind = kKindFp8Fp4, bool kAlwaysStaged = false, bool kPair = false>
 struct GemmSmem {
     static constexpr int kSfIntsPerRow = kKind == kKindNvfp4 ? 4 : 1;  // packed scale ints per row per K block
     static constexpr int kABytes = 128 * 128;
-    static constexpr int kBBytes = BLOCK_N * 128;
+    static constexpr int kBBytes = BLOCK_N * 128 / (kPair ? 2 : 1);  // a pair's CTAs hold half of the tile's channels each
     static constexpr int kSfaBytes = 128 * 4 * kSfIntsPerRow;
     static constexpr int kSfbBytes = BLOCK_N * 4 * kSfIntsPerRow;
     static constexpr int kOffA = 0;
@@ -296,13 +323,13 @@ struct GemmSmem {
     static constexpr int kOffSfa = kOffB + kStages * kBBytes;
     static constexpr int kOffSfb = kOffSfa + kStages * kSfaBytes;
     static constexpr int kOffBar = kOffSfb + kStages * kSfbBytes;
-    static constexpr int kNumBars = 3 * kStages + 4;
+    static constexpr int kNumBars = (kPair ? 4 : 3) * kStages + 4;
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;
     static constexpr int kOffGroups = kOffMisc + 16;
     // Epilogue staging for TMA stores: 32 rows x 64 bytes per epilogue warp, in the 64-byte swizzle (512-byte atoms).
     // The NVFP4 kind only has room for it next to its larger scale-factor stages with 3 pipeline stages.
     static constexpr int kStageBytesPerWarp =
-        (kAlwaysStaged || (BLOCK_N == 256 && (kKind != kKindNvfp4 || kStages <= 3))) ? 2048 : 0;
+        (kAlwaysStaged || kPair || (BLOCK_N == 256 && (kKind != kKindNvfp4 || kStages <= 3))) ? 2048 : 0;
     static constexpr int kOffStage = (kOffGroups + 3 * kMaxCachedGroups * 4 + 511) / 512 * 512;
     static constexpr int kTotal = kOffStage + 8 * kStageBytesPerWarp;
     static constexpr int kDynamicBytes = kTotal + 1024;  // slack to align the base to 1024 B
@@ -325,15 +352,24 @@ constexpr int kGemmThreads = 384;       // warps 0-3: loaders / MMA / transposer
 constexpr int kRegsControlWarps = 96;   // after setmaxnreg: the control warpgroup gives registers away ...
 constexpr int kRegsEpilogueWarps = 200; // ... to the two epilogue warpgroups, which hold a drained accumulator
 
-template <int BLOCK_N, int kStages, int kEpilogue, int kKind = kKindFp8Fp4>
+// kPair: the same kernel on clusters of two CTAs (tcgen05.mma.cta_group::2, a 256 x 256 tile per pair). Each CTA loads its own 128
+// rows of A and HALF of the tile's channels of B with ordinary per-CTA TMA loads that complete on the even CTA's barrier
+// (nothing is multicast); both tensor cores read both halves. What bounds the single-CTA form with byte-wide (or BF16, or
+// NVFP4) weights is the operand bytes an SM takes from L2: 48 KB per K block, 96 bytes per cycle at full tensor rate against
+// about 60 it can get. A pair needs 32 KB per SM, and the smaller stages make the ring deeper (6 instead of 4 stages).
+template <int BLOCK_N, int kStages, int kEpilogue, int kKind = kKindFp8Fp4, bool kPair = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                            const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb,
                            const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ GemmParams p) {
     constexpr bool kPushes = kEpilogue == kEpiSwiGLUPush;
     constexpr int EPI = kPushes ? static_cast<int>(kEpiSwiGLU) : kEpilogue;
-    using L = GemmSmem<BLOCK_N, kStages, kKind, EPI == kEpiF32Acc>;
+    using L = GemmSmem<BLOCK_N, kStages, kKind, EPI == kEpiF32Acc, kPair>;
+    using Sched = TileScheduler<BLOCK_N, EPI == kEpiF32Acc, kPair>;
+    constexpr int kCtas = kPair ? 2 : 1;
+    constexpr int kBRows = BLOCK_N / kCtas;  // channels of B in this CTA's shared memory
     static_assert(BLOCK_N == 128 || BLOCK_N == 256, "BLOCK_N must be 128 or 256");
+    static_assert(!kPair || BLOCK_N == 256, "pairs work on 256 x 256 tiles");
     static_assert(L::kDynamicBytes <= 232448, "shared memory budget");
     constexpr int kSfInts = L::kSfIntsPerRow;          // scale ints per row per K block = tcgen05.cp blocks per 128 rows
     constexpr int kSfBlocksA = kSfInts;                // 512-byte blocks of A scales per stage
@@ -342,10 +378,11 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     constexpr int kTmaXPerKb = kKind == kKindBf16 ? 64 : 128;  // tensor-map elements along K per stage (bytes, 4-bit or 16-bit elements)
     constexpr bool kScaled = kKind != kKindBf16;
     constexpr uint32_t kAccumCols = BLOCK_N;
-    constexpr uint32_t kNumAccum = BLOCK_N == 128 ? 2 : 1;
+    // two accumulators where they fit next to the scale factors (a BF16 tile needs none)
+    constexpr uint32_t kNumAccum = (BLOCK_N == 128 || !kScaled) ? 2 : 1;
     // Scale factors get their own TMEM columns per pipeline stage: with a single region every tcgen05.cp would have
     // to wait for the previous K block's MMAs to finish reading it, which serialises copy and MMA.
-    constexpr uint32_t kSfColsPerStage = 4 * (kSfBlocksA + kSfBlocksB);
+    constexpr uint32_t kSfColsPerStage = kScaled ? 4 * (kSfBlocksA + kSfBlocksB) : 0;
     constexpr uint32_t kSfCol0 = kAccumCols * kNumAccum;
     constexpr uint32_t kTmemCols = 512;
     static_assert(kSfCol0 + kStages * kSfColsPerStage <= kTmemCols, "TMEM budget");
@@ -362,22 +399,29 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     uint64_t* sf_ready_bar = bars + 2 * kStages;
     uint64_t* tmem_full_bar = bars + 3 * kStages;
     uint64_t* tmem_empty_bar = bars + 3 * kStages + 2;
+    uint64_t* sf_full_bar = bars + 3 * kStages + 4;  // pairs only: this CTA's scale factors, see sf_local
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 4);
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
+    const uint32_t cta_rank = kPair ? cluster_cta_rank() : 0u;
+    const bool leader_cta = cta_rank == 0;
+    // Pairs: scale factors in plain row order are transposed by a warp of the CTA they landed in, so they complete on a
+    // barrier of that CTA; everything else completes on the leader's barriers, where the MMA issuer waits.
+    const bool sf_local = kPair && kScaled && p.sf_transposed == 0;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(full_bar + i, 2);       // the A-side loader and the B-side loader
-            mbar_init(empty_bar + i, 1);      // tcgen05.commit of the MMA issuer
-            mbar_init(sf_ready_bar + i, 1);   // one lane of the transposer warp, after a warp barrier
+            mbar_init(full_bar + i, 2 * kCtas);  // the A-side loader and the B-side loader of every CTA
+            mbar_init(empty_bar + i, 1);         // tcgen05.commit of the MMA issuer
+            mbar_init(sf_ready_bar + i, sf_local ? 2 : 1);  // one lane of each transposer warp, after a warp barrier
+            if constexpr (kPair) mbar_init(sf_full_bar + i, 2);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(tmem_full_bar + i, 1);
-            mbar_init(tmem_empty_bar + i, 8);  // lane 0 of each epilogue warp
+            mbar_init(tmem_empty_bar + i, 8 * kCtas);  // lane 0 of each epilogue warp
         }
         fence_mbar_init();
         prefetch_tensormap(&tm_a);
@@ -420,10 +464,10 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     } else if (cache_groups) {
         for (int i = threadIdx.x; i < p.num_groups; i += kGemmThreads) {
             int start, rows, rows_store;
-            TileScheduler<BLOCK_N, EPI == kEpiF32Acc>::group_extent(p, p.layout, i, start, rows, rows_store);
+            Sched::group_extent(p, p.layout, i, start, rows, rows_store);
             group_cache[i] = __ldg(p.layout + i);
             group_start[i] = start;
-            group_tiles_end[i] = (group_selected(p, rows) && group_in_range(p, i)) ? (max(rows, rows_store) + 127) / 128 * (p.n / BLOCK_N) : 0;
+            group_tiles_end[i] = (group_selected(p, rows) && group_in_range(p, i)) ? (max(rows, rows_store) + Sched::kTileM - 1) / Sched::kTileM * (p.n / BLOCK_N) : 0;
         }
         __syncthreads();
         if (warp == 0) {
@@ -445,11 +489,44 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         }
     }
     const GroupTable group_layout{cache_groups ? group_cache : p.layout, group_start, group_tiles_end, cache_groups};
-    if (warp == 2) tmem_alloc(tmem_ptr_smem, kTmemCols);
+    if constexpr (kPair) cluster_sync_all();  // both CTAs run and see each other's initialised barriers
+    if (warp == 2) {
+        if constexpr (kPair) tmem_alloc_pair(tmem_ptr_smem, kTmemCols);
+        else tmem_alloc(tmem_ptr_smem, kTmemCols);
+    }
     tcgen05_fence_before();
     __syncthreads();
+    if constexpr (kPair) cluster_sync_all();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
+
+    // The loads of one stage: which barrier they complete on, and the loader's arrival with its bytes. In a pair the leader's
+    // loader announces the bytes of both CTAs (their loads are alike), the other CTA's loader only arrives.
+    auto stage_arrive = [&](uint32_t stage, uint32_t bytes) {
+        if constexpr (kPair) {
+            if (leader_cta) mbar_arrive_expect_tx(full_bar + stage, 2 * bytes);
+            else mbar_arrive_cluster(map_to_cta(smem_u32(full_bar + stage), 0));
+        } else {
+            mbar_arrive_expect_tx(full_bar + stage, bytes);
+        }
+    };
+    auto load_tile = [&](int smem_off, const CUtensorMap* map, uint32_t stage, int x, int y) {
+        if constexpr (kPair) tma_load_2d_pair(smem + smem_off, map, map_to_cta(smem_u32(full_bar + stage), 0), x, y);
+        else tma_load_2d(smem + smem_off, map, full_bar + stage, x, y);
+    };
+    // a scale-factor load, or its absence in this K block
+    auto load_sf = [&](bool present, uint32_t bytes, int smem_off, const CUtensorMap* map, uint32_t stage, int x, int y) {
+        if (sf_local) {
+            if (present) {
+                mbar_arrive_expect_tx(sf_full_bar + stage, bytes);
+                tma_load_2d(smem + smem_off, map, sf_full_bar + stage, x, y);
+            } else {
+                mbar_arrive(sf_full_bar + stage);
+            }
+        } else if (present) {
+            load_tile(smem_off, map, stage, x, y);
+        }
+    };
 
     const int num_kb = p.k / kBlockK;
     const int a_per = (kKind == kKindNvfp4 || p.gran_a == 32) ? 1 : 4;  // K blocks covered by one packed SF int
@@ -467,7 +544,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         // instructions take their descriptors from uniform registers, which a single-lane (divergent) loop would
         // have to refill through slow register-to-uniform moves for every instruction.
         {
-            TileScheduler<BLOCK_N, EPI == kEpiF32Acc> sched(p, group_layout);
+            Sched sched(p, group_layout);
             Tile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
@@ -480,25 +557,22 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                     if (!ok) break;
                     const bool load_sfa = kScaled && kb % a_per == 0;
                     if (elect_one()) {
-                        mbar_arrive_expect_tx(full_bar + stage, L::kABytes + (load_sfa ? L::kSfaBytes : 0));
+                        stage_arrive(stage, L::kABytes + (load_sfa && !sf_local ? L::kSfaBytes : 0));
+                        const int a_off = L::kOffA + stage * L::kABytes;
                         if constexpr (kKG) {
                             // MN-major A: one box per 128 bytes of M (128 E4M3 or 64 BF16 channels) x kBlockK K rows
                             constexpr int kBoxes = kKind == kKindBf16 ? 2 : 1;
 #pragma unroll
                             for (int h = 0; h < kBoxes; ++h)
-                                tma_load_2d(smem + L::kOffA + stage * L::kABytes + h * (L::kABytes / kBoxes), &tm_a,
-                                            full_bar + stage, t.row_start + h * (128 / kBoxes), t.k_row_start + kb * kBlockK);
+                                load_tile(a_off + h * (L::kABytes / kBoxes), &tm_a, stage, t.row_start + h * (128 / kBoxes),
+                                          t.k_row_start + kb * kBlockK);
                         } else if (kKind == kKindBf16 && p.a_mn_major) {
 #pragma unroll
-                            for (int h = 0; h < 2; ++h)
-                                tma_load_2d(smem + L::kOffA + stage * L::kABytes + h * 8192, &tm_a, full_bar + stage,
-                                            t.row_start + h * 64, kb * 64);
+                            for (int h = 0; h < 2; ++h) load_tile(a_off + h * 8192, &tm_a, stage, t.row_start + h * 64, kb * 64);
                         } else
-                            tma_load_2d(smem + L::kOffA + stage * L::kABytes, &tm_a, full_bar + stage, kb * kTmaXPerKb,
-                                        t.row_start);
-                        if (load_sfa)
-                            tma_load_2d(smem + L::kOffSfa + stage * L::kSfaBytes, &tm_sfa, full_bar + stage,
-                                        t.sf_row_start, sfa_y + kb * kSfInts / a_per);
+                            load_tile(a_off, &tm_a, stage, kb * kTmaXPerKb, t.row_start);
+                        load_sf(load_sfa, L::kSfaBytes, L::kOffSfa + stage * L::kSfaBytes, &tm_sfa, stage, t.sf_row_start,
+                                sfa_y + kb * kSfInts / a_per);
                     }
                     __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -508,7 +582,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     } else if (warp == 3) {
         // ---------------------------------------------------------------- loader: B (weight) tile + its scale factors
         {
-            TileScheduler<BLOCK_N, EPI == kEpiF32Acc> sched(p, group_layout);
+            Sched sched(p, group_layout);
             Tile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
@@ -517,7 +591,6 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
 
             while (ok && sched.next(t)) {
                 if (t.group < 0) continue;
-                const int b_row = t.group * p.n + t.n_block * BLOCK_N;
                 const int sfb_y = kKG ? t.sf_kp0 : t.group * p.sfb_packed_k;
                 const int tile_kb = kKG ? t.num_kb : num_kb;
                 for (int kb = 0; kb < tile_kb; ++kb) {
@@ -525,56 +598,63 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                     if (!ok) break;
                     const bool load_sfb = kScaled && kb % b_per == 0;
                     if (leader) {
-                        mbar_arrive_expect_tx(full_bar + stage, p.b_tx_bytes + (load_sfb ? L::kSfbBytes : 0));
+                        stage_arrive(stage, p.b_tx_bytes + (load_sfb && !sf_local ? L::kSfbBytes : 0));
+                        const int b_off = L::kOffB + stage * L::kBBytes;
+                        const int b_col = t.n_block * BLOCK_N + static_cast<int>(cta_rank) * kBRows;  // first channel of this CTA
                         if constexpr (kKG) {
                             // one box per 128 bytes of N (a swizzle span: 128 E4M3 or 64 BF16 channels) x kBlockK K rows
                             constexpr int kChan = kKind == kKindBf16 ? 64 : 128;
 #pragma unroll
-                            for (int h = 0; h < BLOCK_N / kChan; ++h)
-                                tma_load_2d(smem + L::kOffB + stage * L::kBBytes + h * (128 * kBlockK), &tm_b, full_bar + stage,
-                                            t.n_block * BLOCK_N + h * kChan, t.k_row_start + kb * kBlockK);
+                            for (int h = 0; h < kBRows / kChan; ++h)
+                                load_tile(b_off + h * (128 * kBlockK), &tm_b, stage, b_col + h * kChan, t.k_row_start + kb * kBlockK);
                         } else if (kKind == kKindBf16 && p.b_mn_major) {
                             // MN-major weights: boxes of 64 channels x 64 K rows, as in the K-grouped form
 #pragma unroll
-                            for (int h = 0; h < BLOCK_N / 64; ++h)
-                                tma_load_2d(smem + L::kOffB + stage * L::kBBytes + h * 8192, &tm_b, full_bar + stage,
-                                            t.n_block * BLOCK_N + h * 64, t.group * p.k + kb * 64);
+                            for (int h = 0; h < kBRows / 64; ++h)
+                                load_tile(b_off + h * 8192, &tm_b, stage, b_col + h * 64, t.group * p.k + kb * 64);
                         } else if (kKind == kKindFp8Fp4 && p.b_mn_major) {
                             // MN-major 8-bit (or 4-bit in byte containers) weights: boxes of 128 channels x 128 K rows
 #pragma unroll
-                            for (int h = 0; h < BLOCK_N / 128; ++h)
-                                tma_load_2d(smem + L::kOffB + stage * L::kBBytes + h * 16384, &tm_b, full_bar + stage,
-                                            t.n_block * BLOCK_N + h * 128, t.group * p.k + kb * 128);
+                            for (int h = 0; h < kBRows / 128; ++h)
+                                load_tile(b_off + h * 16384, &tm_b, stage, b_col + h * 128, t.group * p.k + kb * 128);
                         } else
-                            tma_load_2d(smem + L::kOffB + stage * L::kBBytes, &tm_b, full_bar + stage, kb * kTmaXPerKb, b_row);
-                        if (load_sfb)
-                            tma_load_2d(smem + L::kOffSfb + stage * L::kSfbBytes, &tm_sfb, full_bar + stage,
-                                        t.n_block * BLOCK_N, sfb_y + kb * kSfInts / b_per);
+                            load_tile(b_off, &tm_b, stage, kb * kTmaXPerKb, t.group * p.n + b_col);
+                        // the scales of all BLOCK_N channels: each CTA's tensor memory holds them
+                        load_sf(load_sfb, L::kSfbBytes, L::kOffSfb + stage * L::kSfbBytes, &tm_sfb, stage, t.n_block * BLOCK_N,
+                                sfb_y + kb * kSfInts / b_per);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 && leader_cta) {
         // ---------------------------------------------------------------- MMA issuer
         // Warp-uniform loop, one elected lane issues (see the loader above).
         {
-        TileScheduler<BLOCK_N, EPI == kEpiF32Acc> sched(p, group_layout);
+        Sched sched(p, group_layout);
         Tile t;
         uint32_t stage = 0, phase = 0, iter = 0;
         const uint32_t idesc = kKG
-            ? ((kKind == kKindBf16 ? make_idesc_bf16_f32(128, BLOCK_N)
-                                   : make_idesc_block_scaled(kFmtE4M3, kFmtE4M3, 128, BLOCK_N, kScaleUE8M0)) |
+            ? ((kKind == kKindBf16 ? make_idesc_bf16_f32(128 * kCtas, BLOCK_N)
+                                   : make_idesc_block_scaled(kFmtE4M3, kFmtE4M3, 128 * kCtas, BLOCK_N, kScaleUE8M0)) |
                (1u << 15) | (1u << 16))  // both operands MN-major
             : kKind == kKindBf16
-            ? (make_idesc_bf16_f32(128, BLOCK_N) | (p.a_mn_major ? (1u << 15) : 0u) | (p.b_mn_major ? (1u << 16) : 0u))
-            : kKind == kKindNvfp4 ? make_idesc_block_scaled(kFmtE2M1_MXF4, kFmtE2M1_MXF4, 128, BLOCK_N, kScaleUE4M3)
-                                  : (make_idesc_block_scaled(kFmtE4M3, p.b_fmt, 128, BLOCK_N, kScaleUE8M0) |
+            ? (make_idesc_bf16_f32(128 * kCtas, BLOCK_N) | (p.a_mn_major ? (1u << 15) : 0u) | (p.b_mn_major ? (1u << 16) : 0u))
+            : kKind == kKindNvfp4 ? make_idesc_block_scaled(kFmtE2M1_MXF4, kFmtE2M1_MXF4, 128 * kCtas, BLOCK_N, kScaleUE4M3)
+                                  : (make_idesc_block_scaled(kFmtE4M3, p.b_fmt, 128 * kCtas, BLOCK_N, kScaleUE8M0) |
                                      (p.b_mn_major ? (1u << 16) : 0u));
         const uint32_t a_base = smem_u32(smem + L::kOffA), b_base = smem_u32(smem + L::kOffB);
         const uint32_t sfa_smem = smem_u32(smem + L::kOffSfa), sfb_smem = smem_u32(smem + L::kOffSfb);
         uint32_t tmem_sfa = 0, tmem_sfb = 0;  // TMEM columns holding the scale factors of the current K block
         const bool leader = elect_one();      // the same lane issues every tcgen05 instruction of this CTA
+        auto commit = [&](uint64_t* bar) {    // arrives on the barrier of every CTA of the pair
+            if constexpr (kPair) tcgen05_commit_pair(bar, 3);
+            else tcgen05_commit(bar);
+        };
+        auto copy_sf = [&](uint32_t col, uint32_t smem_addr) {
+            if constexpr (kPair) tcgen05_cp_32x128b_warpx4_pair(col, make_sf_desc(smem_addr));
+            else tcgen05_cp_32x128b_warpx4(col, make_sf_desc(smem_addr));
+        };
         bool ok = true;
         while (ok && sched.next(t)) {
             if (t.group < 0) continue;
@@ -585,12 +665,18 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             tcgen05_fence_after();
             const uint32_t tmem_acc = tmem_base + as * kAccumCols;
             const int tile_kb = kKG ? t.num_kb : num_kb;
-            if (kKG && tile_kb == 0 && leader) tcgen05_commit(tmem_full_bar + as);  // empty group: D = C, nothing to wait for
+            if (kKG && tile_kb == 0 && leader) commit(tmem_full_bar + as);  // empty group: D = C, nothing to wait for
             for (int kb = 0; kb < tile_kb; ++kb) {
                 // scale factors stored in tcgen05.cp order need no transposer pass: the loads' barrier is enough
                 ok = mbar_wait(((!kScaled || (p.sf_transposed && !kCpByHelper)) ? full_bar : sf_ready_bar) + stage, phase, abort_flag,
                                kTimeoutSfReady, kb);
                 if (!ok) break;
+                if constexpr (kPair && kScaled) {
+                    if (sf_local) {  // the transposers only waited for the scale factors
+                        ok = mbar_wait(full_bar + stage, phase, abort_flag, kTimeoutFull, kb);
+                        if (!ok) break;
+                    }
+                }
                 if (kCpByHelper && p.sf_transposed) tcgen05_fence_after();  // the helper warp's tcgen05.cp precede our MMAs
                 // No tcgen05 fence here: the data this wait covers was written to shared memory through the async proxy
                 // (TMA, or the transposer's stores followed by its proxy fence), not by tcgen05 operations.
@@ -603,7 +689,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         if (cp_here) {
 #pragma unroll
                             for (int b = 0; b < kSfBlocksA; ++b)
-                                tcgen05_cp_32x128b_warpx4(tmem_sfa + b * 4, make_sf_desc(sfa_smem + stage * L::kSfaBytes + b * 512));
+                                copy_sf(tmem_sfa + b * 4, sfa_smem + stage * L::kSfaBytes + b * 512);
                         }
                     }
                     if (kb % b_per == 0) {
@@ -611,7 +697,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         if (cp_here) {
 #pragma unroll
                             for (int b = 0; b < kSfBlocksB; ++b)
-                                tcgen05_cp_32x128b_warpx4(tmem_sfb + b * 4, make_sf_desc(sfb_smem + stage * L::kSfbBytes + b * 512));
+                                copy_sf(tmem_sfb + b * 4, sfb_smem + stage * L::kSfbBytes + b * 512);
                         }
                     }
                     // MN-major tiles: consecutive 128-byte chunks along M / N are one TMA box (128 bytes x kBlockK rows) apart
@@ -631,21 +717,33 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         // +32 bytes along K inside the 128-byte swizzle span = +2 in the (addr >> 4) field
                         if constexpr (kKind == kKindBf16) {
                             // K = 16 BF16 elements (32 bytes) per MMA
-                            tcgen05_mma_f16(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, (kb | k4) != 0 ? 1u : 0u);
+                            if constexpr (kPair)
+                                tcgen05_mma_f16_pair(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, (kb | k4) != 0 ? 1u : 0u);
+                            else
+                                tcgen05_mma_f16(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, (kb | k4) != 0 ? 1u : 0u);
                         } else if constexpr (kKind == kKindNvfp4) {
                             // K = 64 per MMA; its 4 scales per row are the 4 bytes of packed int k4 of the stage
-                            tcgen05_mma_mxf4nvf4_4x(tmem_acc, adesc + k4 * 2, bdesc + k4 * 2, idesc, tmem_sfa + k4 * 4,
-                                                    tmem_sfb + k4 * (BLOCK_N / 32), (kb | k4) != 0 ? 1u : 0u);
+                            if constexpr (kPair)
+                                tcgen05_mma_mxf4nvf4_4x_pair(tmem_acc, adesc + k4 * 2, bdesc + k4 * 2, idesc, tmem_sfa + k4 * 4,
+                                                             tmem_sfb + k4 * (BLOCK_N / 32), (kb | k4) != 0 ? 1u : 0u);
+                            else
+                                tcgen05_mma_mxf4nvf4_4x(tmem_acc, adesc + k4 * 2, bdesc + k4 * 2, idesc, tmem_sfa + k4 * 4,
+                                                        tmem_sfb + k4 * (BLOCK_N / 32), (kb | k4) != 0 ? 1u : 0u);
                         } else {
                             const uint32_t sfa_id = p.gran_a == 32 ? k4 : static_cast<uint32_t>(kb % 4);
                             const uint32_t sfb_id = p.gran_b == 32 ? k4 : static_cast<uint32_t>(kb % 4);
-                            tcgen05_mma_mxf8f6f4(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step,
-                                                 idesc_with_sf_ids(idesc, sfa_id, sfb_id), tmem_sfa, tmem_sfb,
-                                                 (kb | k4) != 0 ? 1u : 0u);
+                            if constexpr (kPair)
+                                tcgen05_mma_mxf8f6f4_pair(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step,
+                                                          idesc_with_sf_ids(idesc, sfa_id, sfb_id), tmem_sfa, tmem_sfb,
+                                                          (kb | k4) != 0 ? 1u : 0u);
+                            else
+                                tcgen05_mma_mxf8f6f4(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step,
+                                                     idesc_with_sf_ids(idesc, sfa_id, sfb_id), tmem_sfa, tmem_sfb,
+                                                     (kb | k4) != 0 ? 1u : 0u);
                         }
                     }
-                    tcgen05_commit(empty_bar + stage);
-                    if (kb == tile_kb - 1) tcgen05_commit(tmem_full_bar + as);
+                    commit(empty_bar + stage);
+                    if (kb == tile_kb - 1) commit(tmem_full_bar + as);
                 }
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
@@ -654,7 +752,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     } else if (warp == 2) {
         // ---------------------------------------------------------------- scale-factor transposer
         // tcgen05.cp 32x128b wants, per 128 rows, 32 rows x 4 words with word j of row r = source row r + 32 j.
-        TileScheduler<BLOCK_N, EPI == kEpiF32Acc> sched(p, group_layout);
+        Sched sched(p, group_layout);
         Tile t;
         uint32_t stage = 0, phase = 0;
         bool ok = kScaled && p.sf_transposed == 0;  // nothing to do when the scale factors arrive in tcgen05.cp order
@@ -662,7 +760,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             if (t.group < 0) continue;
             const int tile_kb = kKG ? t.num_kb : num_kb;
             for (int kb = 0; kb < tile_kb; ++kb) {
-                ok = mbar_wait(full_bar + stage, phase, abort_flag, kTimeoutFull, kb);
+                ok = mbar_wait((sf_local ? sf_full_bar : full_bar) + stage, phase, abort_flag, kTimeoutFull, kb);
                 if (!ok) break;
                 // All reads first, one warp barrier, then all writes: this warp serves every K block in turn, so its
                 // service time bounds the whole pipeline.
@@ -695,14 +793,21 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(sf_ready_bar + stage);
+                if (lane == 0) {
+                    if (leader_cta) mbar_arrive(sf_ready_bar + stage);
+                    else mbar_arrive_cluster(map_to_cta(smem_u32(sf_ready_bar + stage), 0));
+                }
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }
-        if (kCpByHelper && p.sf_transposed != 0) {
-            TileScheduler<BLOCK_N, EPI == kEpiF32Acc> cp_sched(p, group_layout);
+        if (kCpByHelper && p.sf_transposed != 0 && leader_cta) {
+            Sched cp_sched(p, group_layout);
             const uint32_t sfa_smem = smem_u32(smem + L::kOffSfa), sfb_smem = smem_u32(smem + L::kOffSfb);
             const bool leader = elect_one();
+            auto copy_sf = [&](uint32_t col, uint32_t smem_addr) {
+                if constexpr (kPair) tcgen05_cp_32x128b_warpx4_pair(col, make_sf_desc(smem_addr));
+                else tcgen05_cp_32x128b_warpx4(col, make_sf_desc(smem_addr));
+            };
             stage = 0;
             phase = 0;
             ok = true;
@@ -715,12 +820,13 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         const uint32_t sf_cols = tmem_base + kSfCol0 + stage * kSfColsPerStage;
 #pragma unroll
                         for (int b = 0; b < kSfBlocksA; ++b)
-                            tcgen05_cp_32x128b_warpx4(sf_cols + b * 4, make_sf_desc(sfa_smem + stage * L::kSfaBytes + b * 512));
+                            copy_sf(sf_cols + b * 4, sfa_smem + stage * L::kSfaBytes + b * 512);
 #pragma unroll
                         for (int b = 0; b < kSfBlocksB; ++b)
-                            tcgen05_cp_32x128b_warpx4(sf_cols + 4 * kSfBlocksA + b * 4,
-                                                      make_sf_desc(sfb_smem + stage * L::kSfbBytes + b * 512));
-                        tcgen05_commit(sf_ready_bar + stage);  // arrives once the copies above have completed
+                            copy_sf(sf_cols + 4 * kSfBlocksA + b * 4, sfb_smem + stage * L::kSfbBytes + b * 512);
+                        // arrives once the copies above have completed
+                        if constexpr (kPair) tcgen05_commit_pair(sf_ready_bar + stage, 1);
+                        else tcgen05_commit(sf_ready_bar + stage);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
@@ -734,7 +840,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         // Each thread first drains its half row of the accumulator into registers and releases the accumulator, so
         // the MMA issuer can start the next tile while the arithmetic and the stores below run.
         constexpr int kCols = BLOCK_N / 2;  // accumulator columns per thread
-        TileScheduler<BLOCK_N, EPI == kEpiF32Acc> sched(p, group_layout);
+        Sched sched(p, group_layout);
         Tile t;
         uint32_t iter = 0;
         const uint32_t q = warp & 3, half = (warp - 4) >> 2;
@@ -822,7 +928,10 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tmem_empty_bar + as);
+            if (lane == 0) {
+                if (leader_cta) mbar_arrive(tmem_empty_bar + as);
+                else mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty_bar + as), 0));
+            }
             // Row-per-thread stores put 32 different cache lines into every store instruction, and the burst of a whole
             // tile keeps the load/store pipe busy long enough to stall the control warps' shared-memory accesses.
             // Staging the warp's 32 x 64-byte slab in shared memory and handing it to TMA costs 4 store wavefronts
@@ -1182,9 +1291,11 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         __nanosleep(100000);
         __syncthreads();
     }
+    if constexpr (kPair) cluster_sync_all();  // the other CTA may still signal barriers of this one or read its shared memory
     if (warp == 2) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        if constexpr (kPair) tmem_dealloc_pair(tmem_base, kTmemCols);
+        else tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
