@@ -3,6 +3,7 @@
 // csrc/apis/{gemm,mega,layout,runtime}.hpp argument checking and csrc/jit_kernels/impls/*.hpp launch glue;
 // there is no JIT: every kernel is compiled ahead of time for sm_100a.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -77,6 +78,43 @@ int launch_gemm(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensor
     return 0;
 }
 
+// The split-K form: `split` CTAs per tile, one cluster each, all tiles at once. `max_clusters` receives how many such clusters
+// the device runs at the same time (asked once per form and size; with `dry` nothing is launched).
+template <int BLOCK_N, int kStages, int EPI, int kKind>
+int launch_gemm_split_k(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_sfa, const CUtensorMap& tm_sfb,
+                        const GemmParams& p, int tiles, int split, bool dry, int* max_clusters, cudaStream_t stream) {
+    using L = GemmSmem<BLOCK_N, kStages, kKind, false, false>;
+    static_assert(kStages * (L::kABytes + L::kBBytes) >= 128 * BLOCK_N * 4, "the operand ring holds the FP32 tile");
+    auto kernel = dgb200_grouped_gemm_kernel<BLOCK_N, kStages, EPI, kKind, false, true>;
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> active[kMaxDevices][4] = {};  // [device][log2 split]; 0 = not asked yet
+    int dev = 0;
+    DGB_CUDA(cudaGetDevice(&dev));
+    DGB_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index %d out of range", dev);
+    const int slot = split == 2 ? 1 : (split == 4 ? 2 : 3);
+    int clusters = active[dev][slot].load(std::memory_order_acquire);
+    if (clusters == 0) {
+        DGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned>(split));
+        cfg.blockDim = dim3(kGemmThreads);
+        cfg.dynamicSmemBytes = L::kDynamicBytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        DGB_CUDA(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
+        active[dev][slot].store(clusters > 0 ? clusters : -1, std::memory_order_release);
+    }
+    *max_clusters = std::max(clusters, 0);
+    if (dry) return 0;
+    DGB_CUDA(launch_kernel_in_clusters(split, kernel, dim3(tiles * split), dim3(kGemmThreads), L::kDynamicBytes, stream, use_pdl(), tm_a, tm_b,
+                                       tm_sfa, tm_sfb, tm_a, p));
+    return 0;
+}
+
 struct GemmCall {
     const void* a;
     const void* b;
@@ -103,6 +141,7 @@ struct GemmCall {
 struct Tuning {
     int swap_ab = -1;  // layer GEMMs: tokens on the UMMA N side (-1 = by expected rows per expert, 0 = never, 1 = always)
     int block_n = 0;  // 0 = automatic
+    int split_k = -1;  // dense GEMMs: -1 = by size (split_k_for), 0 = never, 2 / 4 / 8 = that many CTAs per tile where the form exists
     int pair = -1;  // GEMMs on CTA pairs: -1 = by size (use_pairs), 0 = never, 1 = wherever the form exists
     int mlp_kernel = -1;  // FP8 x FP4 layer GEMMs: 0 = separate gate/up and down kernels (tokens-on-M / swapped split),
                           // 1 = the fused expert-MLP kernel on single CTAs, 2 = on CTA pairs; -1 = not yet read from
@@ -161,6 +200,51 @@ bool use_pairs(const GemmCall& c, int block_n, int sms) {
     return c.expected_rows >= (p.mode == kModePsum ? 768 : 512);
 }
 
+template <int BLOCK_N, int kStages>
+int launch_split_k(const GemmCall& c, const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_sfa, const CUtensorMap& tm_sfb,
+                   int tiles, int split, bool dry, int* max_clusters, cudaStream_t stream) {
+    const bool f32 = c.epilogue == kEpiF32;
+    if (c.kind == kKindBf16)
+        return f32 ? launch_gemm_split_k<BLOCK_N, kStages, kEpiF32, kKindBf16>(tm_a, tm_b, tm_sfa, tm_sfb, c.p, tiles, split, dry, max_clusters, stream)
+                   : launch_gemm_split_k<BLOCK_N, kStages, kEpiBF16, kKindBf16>(tm_a, tm_b, tm_sfa, tm_sfb, c.p, tiles, split, dry, max_clusters, stream);
+    return f32 ? launch_gemm_split_k<BLOCK_N, kStages, kEpiF32, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, c.p, tiles, split, dry, max_clusters, stream)
+               : launch_gemm_split_k<BLOCK_N, kStages, kEpiBF16, kKindFp8Fp4>(tm_a, tm_b, tm_sfa, tm_sfb, c.p, tiles, split, dry, max_clusters, stream);
+}
+
+// CTAs per tile of a dense GEMM (1: no split) and the tile width that goes with it: the largest of 8, 4 and 2 for which all
+// clusters run at once and every part keeps at least 8 (12 where more than 64 rows have to be summed) K blocks, the sum over the
+// cluster costing about 3 us. Device time, unsplit -> split (us): BF16 128 x 7168 x 16384 97.7 -> 50.8 (4), 8 x 8192 x 8192 50.6 ->
+// 27.0 (4), 33 x 1536 x 7168 37.2 -> 11.2 (8), 1024 x 2048 x 7168 40.3 -> 30.0 (2); FP8 128 x 7168 x 16384 61.7 -> 36.8 (4), 128 x
+// 2048 x 7168 25.5 -> 15.8 (4). With less K it does not pay: FP8 128 x 4096 x 2048 12.8 -> 14.5 (2).
+int split_k_for(const GemmCall& c, int sms, int* block_n, int* split) {
+    const GemmParams& p = c.p;
+    *split = 1;
+    if (p.mode != kModeDense || (c.kind != kKindBf16 && c.kind != kKindFp8Fp4) || (c.epilogue != kEpiBF16 && c.epilogue != kEpiF32)) return 0;
+    if (tuning().split_k == 0 || tuning().block_n != 0) return 0;
+    const int units = (p.k / (c.kind == kKindBf16 ? 64 : 128) + 3) / 4;
+    const long long m_blocks = (p.m + 127) / 128;
+    const CUtensorMap none{};
+    // the narrow tile only where the wide one could not occupy half of the SMs in clusters of 8
+    const bool narrow = p.n % 256 != 0 || m_blocks * (p.n / 256) * 16 <= sms;
+    for (int bn : {narrow ? 128 : 256, 256}) {
+        if (p.n % bn != 0) continue;
+        const long long tiles = m_blocks * (p.n / bn);
+        for (int s : {8, 4, 2}) {
+            if (tuning().split_k > 0 ? s != tuning().split_k || units < s : units < 8 || units < (p.m > 64 ? 3 : 2) * s) continue;
+            if (tiles * s > sms) continue;
+            int clusters = 0;
+            const int rc = bn == 256 ? launch_split_k<256, 4>(c, none, none, none, none, 0, s, true, &clusters, nullptr)
+                                     : launch_split_k<128, 6>(c, none, none, none, none, 0, s, true, &clusters, nullptr);
+            if (rc) return rc;
+            if (tiles > clusters) continue;
+            *block_n = bn;
+            *split = s;
+            return 0;
+        }
+    }
+    return 0;
+}
+
 int run_gemm(GemmCall& c, cudaStream_t stream) {
     GemmParams& p = c.p;
     const bool nvfp4 = c.kind == kKindNvfp4;
@@ -216,12 +300,14 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     const bool swiglu = c.epilogue == kEpiSwiGLU || c.epilogue == kEpiSwiGLUNvfp4 || c.epilogue == kEpiSwiGLUBf16;
     // the SwiGLU epilogues pair the two 128-channel halves of a 256-wide tile (gate | up)
     DGB_REQUIRE(!swiglu || p.n % 256 == 0, "the gate/up GEMM needs n (%d) to be a multiple of 256", p.n);
-    const int block_n = swiglu ? 256 : (tuning().block_n != 0 ? tuning().block_n : (p.n % 256 == 0 ? 256 : 128));
+    int block_n = swiglu ? 256 : (tuning().block_n != 0 ? tuning().block_n : (p.n % 256 == 0 ? 256 : 128));
     DGB_REQUIRE((block_n == 128 || block_n == 256) && p.n % block_n == 0, "block_n %d does not divide n %d", block_n, p.n);
     int sms = 0;
     rc = effective_num_sms(&sms);
     if (rc) return rc;
-    const bool pair = use_pairs(c, block_n, sms);
+    int split = 1;
+    if ((rc = split_k_for(c, sms, &block_n, &split))) return rc;
+    const bool pair = split == 1 && use_pairs(c, block_n, sms);
     if (!bf16) {
         rc = make_tensor_map_2d(&tm_sfb, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfb, static_cast<uint64_t>(c.sfb_k_stride),
                                 static_cast<uint64_t>(packed_k_b) * p.num_groups, static_cast<uint64_t>(c.sfb_k_stride) * 4,
@@ -290,6 +376,13 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
         p.b_tx_bytes = BLOCK_N * 128;
     }
     if (rc) return rc;
+
+    if (split > 1) {
+        const int tiles = (p.m + 127) / 128 * (p.n / block_n);
+        int clusters = 0;
+        return block_n == 256 ? launch_split_k<256, 4>(c, tm_a, tm_b, tm_sfa, tm_sfb, tiles, split, false, &clusters, stream)
+                              : launch_split_k<128, 6>(c, tm_a, tm_b, tm_sfa, tm_sfb, tiles, split, false, &clusters, stream);
+    }
 
     // Output tensor map for the staged (shared memory + TMA) epilogue stores of the 256-wide FP8 x FP4 kernels.
     CUtensorMap tm_out = tm_a;
@@ -1560,6 +1653,9 @@ int dgb200_set_tuning(const char* name, int32_t value) {
     } else if (std::strcmp(name, "block_n") == 0) {
         DGB_REQUIRE(value == 0 || value == 128 || value == 256, "block_n must be 0 (automatic), 128 or 256");
         tuning().block_n = value;
+    } else if (std::strcmp(name, "split_k") == 0) {
+        DGB_REQUIRE(value == -1 || value == 0 || value == 2 || value == 4 || value == 8, "split_k must be -1 (automatic), 0 (never), 2, 4 or 8");
+        tuning().split_k = value;
     } else if (std::strcmp(name, "pair") == 0) {
         DGB_REQUIRE(value >= -1 && value <= 1, "pair must be -1 (automatic), 0 (never) or 1 (wherever the form exists)");
         tuning().pair = value;

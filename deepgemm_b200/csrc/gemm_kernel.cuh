@@ -32,6 +32,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include <type_traits>
+
 #include "ptx.cuh"
 
 namespace dgb {
@@ -194,6 +196,7 @@ __device__ __forceinline__ bool group_selected(const GemmParams& p, int rows) {
 
 // kPair: a tile is 256 rows tall and belongs to a cluster of two CTAs, each of which sees its own 128 rows (rows_store may
 // then be zero or negative for the second one, which still takes part in the tile's MMAs).
+// `ctas`: CTAs that share a tile (a pair, or a cluster that splits the tile's K).
 template <int BLOCK_N, bool kKGrouped = false, bool kPair = false>
 struct TileScheduler {
     static constexpr int kTileM = kPair ? 256 : 128;
@@ -205,9 +208,9 @@ struct TileScheduler {
     int sub;     // first row of this CTA inside the tile
     int g, tiles_before_g;
 
-    __device__ TileScheduler(const GemmParams& params, const GroupTable& table)
-        : p(params), tab(table), num_n_blocks(params.n / BLOCK_N), tile(static_cast<int>(blockIdx.x) / (kPair ? 2 : 1)),
-          stride(static_cast<int>(gridDim.x) / (kPair ? 2 : 1)), sub(kPair ? static_cast<int>(blockIdx.x & 1) * 128 : 0), g(0),
+    __device__ TileScheduler(const GemmParams& params, const GroupTable& table, int ctas)
+        : p(params), tab(table), num_n_blocks(params.n / BLOCK_N), tile(static_cast<int>(blockIdx.x) / ctas),
+          stride(static_cast<int>(gridDim.x) / ctas), sub(kPair ? static_cast<int>(blockIdx.x & 1) * 128 : 0), g(0),
           tiles_before_g(0) {}
 
     // First row, valid rows and rows to store of one group, from the layout words.
@@ -357,7 +360,12 @@ constexpr int kRegsEpilogueWarps = 200; // ... to the two epilogue warpgroups, w
 // (nothing is multicast); both tensor cores read both halves. What bounds the single-CTA form with byte-wide (or BF16, or
 // NVFP4) weights is the operand bytes an SM takes from L2: 48 KB per K block, 96 bytes per cycle at full tensor rate against
 // about 60 it can get. A pair needs 32 KB per SM, and the smaller stages make the ring deeper (6 instead of 4 stages).
-template <int BLOCK_N, int kStages, int kEpilogue, int kKind = kKindFp8Fp4, bool kPair = false>
+// kSplitK (dense mode): the CTAs of a cluster (2, 4 or 8) share ONE tile and take a part of its K each; every CTA leaves its FP32
+// accumulator in its own shared memory (the operand ring is done with) and then sums, rank by rank in a fixed order, one
+// slice of the tile's rows over the cluster. For problems with so few tiles that most SMs would idle while a few pull all of
+// B: 128 x 7168 x 16384 in BF16 is 28 tiles on 148 SMs: 98 us, with
+// four CTAs per tile 51 (its bytes at the copy rate: 37).
+template <int BLOCK_N, int kStages, int kEpilogue, int kKind = kKindFp8Fp4, bool kPair = false, bool kSplitK = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                            const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb,
@@ -407,6 +415,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t cta_rank = kPair ? cluster_cta_rank() : 0u;
     const bool leader_cta = cta_rank == 0;
+    const int tile_ctas = kPair ? 2 : (kSplitK ? static_cast<int>(cluster_num_ctas()) : 1);
     // Pairs: scale factors in plain row order are transposed by a warp of the CTA they landed in, so they complete on a
     // barrier of that CTA; everything else completes on the leader's barriers, where the MMA issuer waits.
     const bool sf_local = kPair && kScaled && p.sf_transposed == 0;
@@ -529,6 +538,13 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     };
 
     const int num_kb = p.k / kBlockK;
+    // this CTA's K blocks, whole groups of 4 (what one packed scale int may cover); the host leaves no part empty
+    int kb_lo = 0, kb_hi = num_kb;
+    if constexpr (kSplitK) {
+        const int rank = static_cast<int>(cluster_cta_rank()), units = (num_kb + 3) / 4;
+        kb_lo = units * rank / tile_ctas * 4;
+        kb_hi = min(units * (rank + 1) / tile_ctas * 4, num_kb);
+    }
     const int a_per = (kKind == kKindNvfp4 || p.gran_a == 32) ? 1 : 4;  // K blocks covered by one packed SF int
     const int b_per = (kKind == kKindNvfp4 || p.gran_b == 32) ? 1 : 4;
 
@@ -544,15 +560,15 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         // instructions take their descriptors from uniform registers, which a single-lane (divergent) loop would
         // have to refill through slow register-to-uniform moves for every instruction.
         {
-            Sched sched(p, group_layout);
+            Sched sched(p, group_layout, tile_ctas);
             Tile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             while (ok && sched.next(t)) {
                 if (t.group < 0) continue;
                 const int sfa_y = kKG ? t.sf_kp0 : t.group * p.sfa_group_rows;
-                const int tile_kb = kKG ? t.num_kb : num_kb;
-                for (int kb = 0; kb < tile_kb; ++kb) {
+                const int tile_kb = kKG ? t.num_kb : kb_hi;
+                for (int kb = kb_lo; kb < tile_kb; ++kb) {
                     ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, kTimeoutEmpty, kb);
                     if (!ok) break;
                     const bool load_sfa = kScaled && kb % a_per == 0;
@@ -582,7 +598,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     } else if (warp == 3) {
         // ---------------------------------------------------------------- loader: B (weight) tile + its scale factors
         {
-            Sched sched(p, group_layout);
+            Sched sched(p, group_layout, tile_ctas);
             Tile t;
             uint32_t stage = 0, phase = 0;
             bool ok = true;
@@ -592,8 +608,8 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             while (ok && sched.next(t)) {
                 if (t.group < 0) continue;
                 const int sfb_y = kKG ? t.sf_kp0 : t.group * p.sfb_packed_k;
-                const int tile_kb = kKG ? t.num_kb : num_kb;
-                for (int kb = 0; kb < tile_kb; ++kb) {
+                const int tile_kb = kKG ? t.num_kb : kb_hi;
+                for (int kb = kb_lo; kb < tile_kb; ++kb) {
                     ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, kTimeoutEmpty, kb);
                     if (!ok) break;
                     const bool load_sfb = kScaled && kb % b_per == 0;
@@ -631,7 +647,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         // ---------------------------------------------------------------- MMA issuer
         // Warp-uniform loop, one elected lane issues (see the loader above).
         {
-        Sched sched(p, group_layout);
+        Sched sched(p, group_layout, tile_ctas);
         Tile t;
         uint32_t stage = 0, phase = 0, iter = 0;
         const uint32_t idesc = kKG
@@ -664,9 +680,9 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t tmem_acc = tmem_base + as * kAccumCols;
-            const int tile_kb = kKG ? t.num_kb : num_kb;
+            const int tile_kb = kKG ? t.num_kb : kb_hi;
             if (kKG && tile_kb == 0 && leader) commit(tmem_full_bar + as);  // empty group: D = C, nothing to wait for
-            for (int kb = 0; kb < tile_kb; ++kb) {
+            for (int kb = kb_lo; kb < tile_kb; ++kb) {
                 // scale factors stored in tcgen05.cp order need no transposer pass: the loads' barrier is enough
                 ok = mbar_wait(((!kScaled || (p.sf_transposed && !kCpByHelper)) ? full_bar : sf_ready_bar) + stage, phase, abort_flag,
                                kTimeoutSfReady, kb);
@@ -718,28 +734,28 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         if constexpr (kKind == kKindBf16) {
                             // K = 16 BF16 elements (32 bytes) per MMA
                             if constexpr (kPair)
-                                tcgen05_mma_f16_pair(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, (kb | k4) != 0 ? 1u : 0u);
+                                tcgen05_mma_f16_pair(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                             else
-                                tcgen05_mma_f16(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, (kb | k4) != 0 ? 1u : 0u);
+                                tcgen05_mma_f16(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step, idesc, ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                         } else if constexpr (kKind == kKindNvfp4) {
                             // K = 64 per MMA; its 4 scales per row are the 4 bytes of packed int k4 of the stage
                             if constexpr (kPair)
                                 tcgen05_mma_mxf4nvf4_4x_pair(tmem_acc, adesc + k4 * 2, bdesc + k4 * 2, idesc, tmem_sfa + k4 * 4,
-                                                             tmem_sfb + k4 * (BLOCK_N / 32), (kb | k4) != 0 ? 1u : 0u);
+                                                             tmem_sfb + k4 * (BLOCK_N / 32), ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                             else
                                 tcgen05_mma_mxf4nvf4_4x(tmem_acc, adesc + k4 * 2, bdesc + k4 * 2, idesc, tmem_sfa + k4 * 4,
-                                                        tmem_sfb + k4 * (BLOCK_N / 32), (kb | k4) != 0 ? 1u : 0u);
+                                                        tmem_sfb + k4 * (BLOCK_N / 32), ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                         } else {
                             const uint32_t sfa_id = p.gran_a == 32 ? k4 : static_cast<uint32_t>(kb % 4);
                             const uint32_t sfb_id = p.gran_b == 32 ? k4 : static_cast<uint32_t>(kb % 4);
                             if constexpr (kPair)
                                 tcgen05_mma_mxf8f6f4_pair(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step,
                                                           idesc_with_sf_ids(idesc, sfa_id, sfb_id), tmem_sfa, tmem_sfb,
-                                                          (kb | k4) != 0 ? 1u : 0u);
+                                                          ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                             else
                                 tcgen05_mma_mxf8f6f4(tmem_acc, adesc + k4 * a_step, bdesc + k4 * b_step,
                                                      idesc_with_sf_ids(idesc, sfa_id, sfb_id), tmem_sfa, tmem_sfb,
-                                                     (kb | k4) != 0 ? 1u : 0u);
+                                                     ((kb - kb_lo) | k4) != 0 ? 1u : 0u);
                         }
                     }
                     commit(empty_bar + stage);
@@ -752,14 +768,14 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     } else if (warp == 2) {
         // ---------------------------------------------------------------- scale-factor transposer
         // tcgen05.cp 32x128b wants, per 128 rows, 32 rows x 4 words with word j of row r = source row r + 32 j.
-        Sched sched(p, group_layout);
+        Sched sched(p, group_layout, tile_ctas);
         Tile t;
         uint32_t stage = 0, phase = 0;
         bool ok = kScaled && p.sf_transposed == 0;  // nothing to do when the scale factors arrive in tcgen05.cp order
         while (ok && sched.next(t)) {
             if (t.group < 0) continue;
-            const int tile_kb = kKG ? t.num_kb : num_kb;
-            for (int kb = 0; kb < tile_kb; ++kb) {
+            const int tile_kb = kKG ? t.num_kb : kb_hi;
+            for (int kb = kb_lo; kb < tile_kb; ++kb) {
                 ok = mbar_wait((sf_local ? sf_full_bar : full_bar) + stage, phase, abort_flag, kTimeoutFull, kb);
                 if (!ok) break;
                 // All reads first, one warp barrier, then all writes: this warp serves every K block in turn, so its
@@ -801,7 +817,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             }
         }
         if (kCpByHelper && p.sf_transposed != 0 && leader_cta) {
-            Sched cp_sched(p, group_layout);
+            Sched cp_sched(p, group_layout, tile_ctas);
             const uint32_t sfa_smem = smem_u32(smem + L::kOffSfa), sfb_smem = smem_u32(smem + L::kOffSfb);
             const bool leader = elect_one();
             auto copy_sf = [&](uint32_t col, uint32_t smem_addr) {
@@ -840,7 +856,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         // Each thread first drains its half row of the accumulator into registers and releases the accumulator, so
         // the MMA issuer can start the next tile while the arithmetic and the stores below run.
         constexpr int kCols = BLOCK_N / 2;  // accumulator columns per thread
-        Sched sched(p, group_layout);
+        Sched sched(p, group_layout, tile_ctas);
         Tile t;
         uint32_t iter = 0;
         const uint32_t q = warp & 3, half = (warp - 4) >> 2;
@@ -908,6 +924,21 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             ok = mbar_wait<32>(tmem_full_bar + as, aphase, abort_flag, kTimeoutTmemFull, static_cast<int>(iter));
             if (!ok) break;
             tcgen05_fence_after();
+            if constexpr (kSplitK) {
+                // the operand ring is free: every load of this CTA has landed and the MMAs that read them have retired
+                uint8_t* mine = smem + r * (BLOCK_N * 4);
+#pragma unroll 1
+                for (int c0 = 0; c0 < kCols; c0 += 32) {
+                    uint32_t v[32];
+                    const int col = static_cast<int>(half) * kCols + c0;
+                    tmem_ld_32x32b_x32(tmem_base + as * kAccumCols + ((q * 32u) << 16) + col, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)  // 16-byte chunks, XOR-swizzled so that 8 rows hit 8 different bank groups
+                        *reinterpret_cast<uint4*>(mine + (((col / 4 + i) ^ (r & 7)) << 4)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                }
+                continue;  // the cluster sums and stores below
+            }
             uint32_t acc[kCols];
             if (warp_has_rows) {
                 if constexpr (EPI == kEpiSwiGLU || EPI == kEpiSwiGLUNvfp4 || EPI == kEpiSwiGLUBf16) {
@@ -1281,6 +1312,62 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         }
         if constexpr (kPushes) push_rows(0x7fffffff);  // whatever is left of this warp's share
         if (L::kStageBytesPerWarp != 0 && lane == 0) bulk_wait_group_all();  // stores still in flight read this CTA's shared memory
+    }
+
+    if constexpr (kSplitK) {
+        // A CTA that gave up on a wait leaves zeros or stale bytes in its part; the error is in the status block.
+        __syncwarp();
+        cluster_sync_all();
+        const int rank = static_cast<int>(cluster_cta_rank());
+        const int slice = 128 / tile_ctas;  // rows of the tile this CTA sums
+        constexpr int kOct = BLOCK_N / 8;   // 8 columns per thread and step
+        Sched sched(p, group_layout, tile_ctas);
+        Tile t;
+        if (sched.next(t)) {
+            for (int i = static_cast<int>(threadIdx.x); i < slice * kOct; i += kGemmThreads) {
+                const int row = rank * slice + i / kOct, oct = i % kOct;
+                if (row >= t.rows_store) continue;
+                float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                const uint32_t at_row = smem_u32(smem + row * (BLOCK_N * 4));
+                // every load of two (or four) ranks in flight before the first sum
+                auto add_ranks = [&](int c0, auto count) {
+                    constexpr int kCount = decltype(count)::value;
+                    float4 f[kCount][2];
+#pragma unroll
+                    for (int c = 0; c < kCount; ++c)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            f[c][h] = ld_cluster_f4(map_to_cta(at_row + (((oct * 2 + h) ^ (row & 7)) << 4), static_cast<uint32_t>(c0 + c)));
+#pragma unroll
+                    for (int c = 0; c < kCount; ++c)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            v[4 * h] += f[c][h].x;
+                            v[4 * h + 1] += f[c][h].y;
+                            v[4 * h + 2] += f[c][h].z;
+                            v[4 * h + 3] += f[c][h].w;
+                        }
+                };
+                if (tile_ctas == 2) add_ranks(0, std::integral_constant<int, 2>{});
+                for (int c = 0; c + 4 <= tile_ctas; c += 4) add_ranks(c, std::integral_constant<int, 4>{});
+                const long long at = (static_cast<long long>(t.row_start) + row) * p.d_row_stride +
+                                     static_cast<long long>(t.n_block) * BLOCK_N + oct * 8;
+                if constexpr (EPI == kEpiBF16) {
+                    st_global_v4(reinterpret_cast<__nv_bfloat16*>(p.d) + at, pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                 pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+                } else {
+                    float* dst = reinterpret_cast<float*>(p.d) + at;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float4 old = make_float4(0, 0, 0, 0);
+                        if (p.accumulate) old = *reinterpret_cast<const float4*>(dst + h * 4);
+                        st_global_v4(dst + h * 4, __float_as_uint(old.x + v[4 * h]), __float_as_uint(old.y + v[4 * h + 1]),
+                                     __float_as_uint(old.z + v[4 * h + 2]), __float_as_uint(old.w + v[4 * h + 3]));
+                    }
+                }
+            }
+        }
+        cluster_sync_all();  // nobody leaves while others read its shared memory
     }
 
     // ---------------------------------------------------------------- teardown
