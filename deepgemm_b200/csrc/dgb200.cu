@@ -556,20 +556,22 @@ int allow_row_mover_smem(Kernel kernel) {
 // The layer GEMMs with swapped operands (gemm_swap_kernel.cuh): weights on M, an expert's tokens on N. Takes the same
 // call description as run_gemm; only the FP8 x FP4 / FP8 x FP8 kind, the psum layout with 128-row segments, scale
 // factors in tcgen05.cp order and the SwiGLU / BF16 epilogues.
-template <int EPI>
-int launch_gemm_swap(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const CUtensorMap& tm_sfx, const CUtensorMap& tm_sfw,
-                     const GemmParams& p, int grid, cudaStream_t stream) {
-    auto kernel = dgb200_swap_gemm_kernel<EPI>;
+template <int EPI, int kSmallTok>
+int launch_gemm_swap(const CUtensorMap& tm_x, const CUtensorMap& tm_xs, const CUtensorMap& tm_w, const CUtensorMap& tm_sfx,
+                     const CUtensorMap& tm_sfxs, const CUtensorMap& tm_sfw, const GemmParams& p, int grid, cudaStream_t stream) {
+    auto kernel = dgb200_swap_gemm_kernel<EPI, kSmallTok>;
+    constexpr int kBytes = SwapSmem<kSmallTok>::kDynamicBytes;
     static bool configured = false;
     static int configured_device = -1;
     int dev = 0;
     DGB_CUDA(cudaGetDevice(&dev));
     if (!configured || configured_device != dev) {
-        DGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SwapSmem::kDynamicBytes));
+        DGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
         configured = true;
         configured_device = dev;
     }
-    DGB_CUDA(launch_kernel(kernel, dim3(grid), dim3(kGemmThreads), SwapSmem::kDynamicBytes, stream, use_pdl(), tm_x, tm_w, tm_sfx, tm_sfw, p));
+    DGB_CUDA(launch_kernel(kernel, dim3(grid), dim3(kGemmThreads), kBytes, stream, use_pdl(), tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs,
+                           tm_sfw, p));
     return 0;
 }
 
@@ -588,15 +590,21 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
                 "scale factors of B: group stride must equal packed K x MN stride");
     p.sfb_packed_k = packed_k;
     if (c.a_rows_total == 0) return 0;
-    CUtensorMap tm_x, tm_w, tm_sfx, tm_sfw;
-    int rc = make_tensor_map_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.a, static_cast<uint64_t>(p.k),
-                                static_cast<uint64_t>(c.a_rows_total), static_cast<uint64_t>(p.k), 128, kSwapMaxTok,
-                                CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    rc = make_tensor_map_2d(&tm_sfx, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfa, static_cast<uint64_t>(c.sfa_k_stride),
-                            static_cast<uint64_t>(packed_k), static_cast<uint64_t>(c.sfa_k_stride) * 4, 256, 1,
-                            CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
+    CUtensorMap tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw;
+    // Token slots of the small ring layout by the rows a group is expected to have: a group that exceeds them changes the
+    // layout, which costs a drained ring, so the line lies where few groups do (10 rows expected: 1 in 40 has more than 16).
+    const bool tiny = c.expected_rows > 0 && c.expected_rows <= 10;
+    int rc = 0;
+    for (int i = 0; i < 2; ++i) {
+        rc = make_tensor_map_2d(i == 0 ? &tm_x : &tm_xs, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.a, static_cast<uint64_t>(p.k),
+                                static_cast<uint64_t>(c.a_rows_total), static_cast<uint64_t>(p.k), 128,
+                                i == 0 ? kSwapMaxTok : (tiny ? 16 : 64), CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc) return rc;
+        rc = make_tensor_map_2d(i == 0 ? &tm_sfx : &tm_sfxs, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfa, static_cast<uint64_t>(c.sfa_k_stride),
+                                static_cast<uint64_t>(packed_k), static_cast<uint64_t>(c.sfa_k_stride) * 4, i == 0 ? 256 : 128, 1,
+                                CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc) return rc;
+    }
     rc = make_tensor_map_2d(&tm_sfw, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfb, static_cast<uint64_t>(c.sfb_k_stride),
                             static_cast<uint64_t>(p.num_groups) * packed_k, static_cast<uint64_t>(c.sfb_k_stride) * 4, 256, 1,
                             CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -617,8 +625,11 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     int sms = 0;
     rc = effective_num_sms(&sms);
     if (rc) return rc;
-    if (c.epilogue == kEpiSwiGLU) return launch_gemm_swap<kEpiSwiGLU>(tm_x, tm_w, tm_sfx, tm_sfw, p, sms, stream);
-    return launch_gemm_swap<kEpiBF16>(tm_x, tm_w, tm_sfx, tm_sfw, p, sms, stream);
+    if (c.epilogue == kEpiSwiGLU)
+        return tiny ? launch_gemm_swap<kEpiSwiGLU, 16>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream)
+                    : launch_gemm_swap<kEpiSwiGLU, 64>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
+    return tiny ? launch_gemm_swap<kEpiBF16, 16>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream)
+                : launch_gemm_swap<kEpiBF16, 64>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
 }
 
 // --------------------------------------------------------------------------------------------------------------
@@ -993,6 +1004,7 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
         c.a_row_stride_bytes = c.b_row_stride_bytes = hidden * 2ll;  // BF16 kind
         c.whole_tile_stores = 1;
         c.max_tiles = 0;
+        c.expected_rows = std::max(expected_rows_per_expert, 1ll);
         c.sfa = base + l.l1_sf;
         c.sfb = l1_w_sf;
         c.sfa_k_stride = l.max_rows;
@@ -1039,6 +1051,7 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
         c.a_row_stride_bytes = c.b_row_stride_bytes = intermediate_hidden * 2ll;  // BF16 kind
         c.whole_tile_stores = 1;
         c.max_tiles = 0;
+        c.expected_rows = std::max(expected_rows_per_expert, 1ll);
         c.sfa = base + l.l2_sf;
         c.sfb = l2_w_sf;
         c.sfa_k_stride = l.max_rows;

@@ -24,24 +24,67 @@
 namespace dgb {
 
 constexpr int kSwapMaxTok = 160;  // tokens per tile = largest UMMA N used (multiple of 16)
-constexpr int kSwapStages = 4;
 
+// The operand ring has two layouts over the same shared memory: tiles of up to kSmallTok tokens use small token slots and more
+// stages, all others slots of kSwapMaxTok tokens and 4 stages. A decode tile is bound by how many bytes of weights an SM has
+// under way: its stage of 256 weight rows is 16 KB of HBM traffic whatever the tokens, and 4 stages (64 KB) do not cover the
+// loaded latency of HBM at full rate (256 tokens over 256 experts, gate/up GEMM: 696 -> 637 us, 5.9 TB/s).
+// Every role walks the same tiles, so each of them changes the layout at the same tile; the loaders first wait until the
+// last stages of the old layout have been consumed.
+template <int kSmallTok>
 struct SwapSmem {
+    static_assert(kSmallTok == 16 || kSmallTok == 64, "token slots of the small layout");
+    static constexpr int kSmallStages = kSmallTok == 16 ? 6 : 5, kLargeStages = 4;
+    static constexpr int kStages = kSmallStages;       // barriers
     static constexpr int kWBytes = 256 * 128;          // 256 weight rows x 128 K bytes (packed FP4 expanded by TMA)
-    static constexpr int kXBytes = kSwapMaxTok * 128;  // token rows x 128 K bytes
     static constexpr int kSfwBytes = 2 * 512;          // one packed scale int per weight row
-    static constexpr int kSfxBytes = 2 * 512;          // one packed scale int per token row (256-row box, 160 used)
-    static constexpr int kOffW = 0;
-    static constexpr int kOffX = kOffW + kSwapStages * kWBytes;
-    static constexpr int kOffSfw = kOffX + kSwapStages * kXBytes;
-    static constexpr int kOffSfx = kOffSfw + kSwapStages * kSfwBytes;
-    static constexpr int kOffBar = kOffSfx + kSwapStages * kSfxBytes;
-    static constexpr int kNumBars = 2 * kSwapStages + 2;
+    static constexpr int kSmallX = kSmallTok * 128, kLargeX = kSwapMaxTok * 128;  // token rows x 128 K bytes
+    static constexpr int kSmallSfx = 512, kLargeSfx = 2 * 512;  // packed scale ints of 128 or 256 token rows
+    static constexpr int kRing = kLargeStages * (kWBytes + kLargeX + kSfwBytes + kLargeSfx);
+    static_assert(kSmallStages * (kWBytes + kSmallX + kSfwBytes + kSmallSfx) <= kRing, "both layouts share the ring");
+    static constexpr int kOffBar = kRing;
+    static constexpr int kNumBars = 2 * kStages + 2;
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;
     static constexpr int kOffGroups = kOffMisc + 16;
     static constexpr int kTotal = kOffGroups + 3 * kMaxCachedGroups * 4;
     static constexpr int kDynamicBytes = kTotal + 1024;
-    static_assert(kXBytes % 1024 == 0, "token tiles must keep the 1024-byte alignment of the 128-byte swizzle");
+    static_assert(kSmallX % 1024 == 0 && kLargeX % 1024 == 0, "token tiles must keep the 1024-byte alignment of the 128-byte swizzle");
+    static_assert(kDynamicBytes <= 232448, "shared memory budget");
+};
+
+// One role's position in the ring: the layout in use, the next stage, and per stage the parity its next use waits for.
+template <int kSmallTok>
+struct SwapRing {
+    using L = SwapSmem<kSmallTok>;
+    bool small = true;
+    int stage = 0;
+    uint32_t parity = 0;  // bit s: parity of stage s's full barrier at its next use (its empty barrier: the opposite)
+
+    __device__ __forceinline__ int stages() const { return small ? L::kSmallStages : L::kLargeStages; }
+    __device__ __forceinline__ uint32_t phase() const { return (parity >> stage) & 1u; }
+    __device__ __forceinline__ void advance() {
+        parity ^= 1u << stage;
+        if (++stage == stages()) stage = 0;
+    }
+    __device__ __forceinline__ int x_bytes() const { return small ? L::kSmallX : L::kLargeX; }
+    __device__ __forceinline__ int sfx_bytes() const { return small ? L::kSmallSfx : L::kLargeSfx; }
+    __device__ __forceinline__ int off_w() const { return stage * L::kWBytes; }
+    __device__ __forceinline__ int off_x() const { return stages() * L::kWBytes + stage * x_bytes(); }
+    __device__ __forceinline__ int off_sfw() const { return stages() * (L::kWBytes + x_bytes()) + stage * L::kSfwBytes; }
+    __device__ __forceinline__ int off_sfx() const { return stages() * (L::kWBytes + x_bytes() + L::kSfwBytes) + stage * sfx_bytes(); }
+    // Takes up the layout of a tile of `tokens` rows. True when it changes: the loaders then drain() before they write.
+    __device__ __forceinline__ bool enter(int tokens) {
+        const bool want = tokens <= kSmallTok;
+        if (want == small) return false;
+        small = want;
+        stage = 0;
+        return true;
+    }
+    __device__ __forceinline__ bool drain(uint64_t* empty_bar, volatile uint32_t* abort_flag) const {
+        for (int s = 0; s < L::kStages; ++s)
+            if (!mbar_wait(empty_bar + s, ((parity >> s) & 1u) ^ 1u, abort_flag, kTimeoutEmpty, s)) return false;
+        return true;
+    }
 };
 
 struct SwapTile {
@@ -69,7 +112,7 @@ struct SwapScheduler {
           tile(static_cast<int>(blockIdx.x)), g(0) {}
 
     __device__ bool next(SwapTile& t) {
-        while (g < num_groups && tile >= tiles_end[g]) ++g;
+        g = group_of_tile(tiles_end, g, num_groups, tile);
         if (g >= num_groups) return false;
         int local = tile - (g == 0 ? 0 : tiles_end[g - 1]);
         const int rows = lay[g] - start[g];
@@ -84,15 +127,16 @@ struct SwapScheduler {
     }
 };
 
-// tm_x: tokens [rows, K] bytes, box 128 x kSwapMaxTok; tm_w: weights (16U4_ALIGN16B) box 128 x 256;
-// tm_sfx / tm_sfw: packed scale ints, box 256 x 1. p: the GemmParams of the layer call (psum layout, alignment 128).
-template <int EPI>
+// tm_x / tm_xs: tokens [rows, K] bytes, box 128 x kSwapMaxTok / kSmallTok; tm_w: weights (16U4_ALIGN16B) box 128 x 256;
+// tm_sfx / tm_sfxs: packed scale ints of the tokens, box 256 / 128 x 1; tm_sfw: of the weights, box 256 x 1. p: the GemmParams of the layer call (psum layout, alignment 128).
+template <int EPI, int kSmallTok>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
-                        const __grid_constant__ CUtensorMap tm_sfx, const __grid_constant__ CUtensorMap tm_sfw,
+dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xs,
+                        const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_sfx,
+                        const __grid_constant__ CUtensorMap tm_sfxs, const __grid_constant__ CUtensorMap tm_sfw,
                         const __grid_constant__ GemmParams p) {
-    using L = SwapSmem;
-    constexpr int kStages = kSwapStages;
+    using L = SwapSmem<kSmallTok>;
+    constexpr int kStages = L::kStages;
     constexpr uint32_t kAcc1Col = kSwapMaxTok;           // accumulator 0: columns [0, 160), accumulator 1: [160, 320)
     constexpr uint32_t kSfCol0 = 2 * kSwapMaxTok;
     constexpr uint32_t kSfColsPerStage = 16;             // weights 2 x 4, tokens 2 x 4
@@ -124,10 +168,13 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         mbar_init(tmem_empty_bar, 8);     // lane 0 of each epilogue warp
         fence_mbar_init();
         prefetch_tensormap(&tm_x);
+        prefetch_tensormap(&tm_xs);
         prefetch_tensormap(&tm_w);
         prefetch_tensormap(&tm_sfx);
+        prefetch_tensormap(&tm_sfxs);
         prefetch_tensormap(&tm_sfw);
     }
+    pdl_prologue();  // everything above touches only this CTA's shared memory and the kernel's own parameters
     // per-group table: layout word, first row, running tile count (host guarantees num_groups <= kMaxCachedGroups)
     int* group_lay = reinterpret_cast<int*>(smem + L::kOffGroups);
     int* group_start = group_lay + kMaxCachedGroups;
@@ -171,49 +218,55 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         // ---------------------------------------------------------------- loader: token rows + their scale ints
         SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
         SwapTile t;
-        uint32_t stage = 0, phase = 0;
+        SwapRing<kSmallTok> ring;
         const bool leader = elect_one();
         bool ok = true;
         while (ok && sched.next(t)) {
-            for (int kb = 0; kb < num_kb; ++kb) {
-                ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, kTimeoutEmpty, kb);
+            if (ring.enter(t.tokens)) ok = ring.drain(empty_bar, abort_flag);
+            const CUtensorMap* x_map = ring.small ? &tm_xs : &tm_x;
+            const CUtensorMap* sfx_map = ring.small ? &tm_sfxs : &tm_sfx;
+            for (int kb = 0; ok && kb < num_kb; ++kb) {
+                ok = mbar_wait(empty_bar + ring.stage, ring.phase() ^ 1, abort_flag, kTimeoutEmpty, kb);
                 if (!ok) break;
                 if (leader) {
-                    mbar_arrive_expect_tx(full_bar + stage, L::kXBytes + L::kSfxBytes);
-                    tma_load_2d(smem + L::kOffX + stage * L::kXBytes, &tm_x, full_bar + stage, kb * 128, t.row_start);
-                    tma_load_2d(smem + L::kOffSfx + stage * L::kSfxBytes, &tm_sfx, full_bar + stage, t.row_start, kb);
+                    uint64_t* bar = full_bar + ring.stage;
+                    mbar_arrive_expect_tx(bar, ring.x_bytes() + ring.sfx_bytes());
+                    tma_load_2d(smem + ring.off_x(), x_map, bar, kb * 128, t.row_start);
+                    tma_load_2d(smem + ring.off_sfx(), sfx_map, bar, t.row_start, kb);
                 }
-                if (++stage == kStages) { stage = 0; phase ^= 1; }
+                ring.advance();
             }
         }
     } else if (warp == 3) {
         // ---------------------------------------------------------------- loader: weight rows + their scale ints
         SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
         SwapTile t;
-        uint32_t stage = 0, phase = 0;
+        SwapRing<kSmallTok> ring;
         const bool leader = elect_one();
         bool ok = true;
         while (ok && sched.next(t)) {
+            if (ring.enter(t.tokens)) ok = ring.drain(empty_bar, abort_flag);
             const int w_row = t.group * p.n + t.w_block * 256;
             const int sfw_y = t.group * p.sfb_packed_k;
-            for (int kb = 0; kb < num_kb; ++kb) {
-                ok = mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, kTimeoutEmpty, kb);
+            for (int kb = 0; ok && kb < num_kb; ++kb) {
+                ok = mbar_wait(empty_bar + ring.stage, ring.phase() ^ 1, abort_flag, kTimeoutEmpty, kb);
                 if (!ok) break;
                 if (leader) {
-                    mbar_arrive_expect_tx(full_bar + stage, p.b_tx_bytes + L::kSfwBytes);
-                    tma_load_2d(smem + L::kOffW + stage * L::kWBytes, &tm_w, full_bar + stage, kb * 128, w_row);
-                    tma_load_2d(smem + L::kOffSfw + stage * L::kSfwBytes, &tm_sfw, full_bar + stage, t.w_block * 256, sfw_y + kb);
+                    uint64_t* bar = full_bar + ring.stage;
+                    mbar_arrive_expect_tx(bar, p.b_tx_bytes + L::kSfwBytes);
+                    tma_load_2d(smem + ring.off_w(), &tm_w, bar, kb * 128, w_row);
+                    tma_load_2d(smem + ring.off_sfw(), &tm_sfw, bar, t.w_block * 256, sfw_y + kb);
                 }
-                if (++stage == kStages) { stage = 0; phase ^= 1; }
+                ring.advance();
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
         SwapTile t;
-        uint32_t stage = 0, phase = 0, iter = 0;
-        const uint32_t w_base = smem_u32(smem + L::kOffW), x_base = smem_u32(smem + L::kOffX);
-        const uint32_t sfw_smem = smem_u32(smem + L::kOffSfw), sfx_smem = smem_u32(smem + L::kOffSfx);
+        uint32_t iter = 0;
+        SwapRing<kSmallTok> ring;
+        const uint32_t smem_base = smem_u32(smem);
         const bool leader = elect_one();
         bool ok = true;
         while (ok && sched.next(t)) {
@@ -221,21 +274,23 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             ++iter;
             if (!ok) break;
             tcgen05_fence_after();
+            (void)ring.enter(t.tokens);
             const uint32_t n_tok = static_cast<uint32_t>((t.tokens + 15) & ~15);
             // weights are the A operand (E2M1 in byte containers or E4M3), tokens the B operand (E4M3)
             const uint32_t idesc = make_idesc_block_scaled(p.b_fmt, kFmtE4M3, 128, n_tok, kScaleUE8M0);
             for (int kb = 0; kb < num_kb; ++kb) {
-                ok = mbar_wait(full_bar + stage, phase, abort_flag, kTimeoutFull, kb);
+                ok = mbar_wait(full_bar + ring.stage, ring.phase(), abort_flag, kTimeoutFull, kb);
                 if (!ok) break;
                 if (leader) {
-                    const uint32_t sf_cols = tmem_base + kSfCol0 + stage * kSfColsPerStage;
+                    const uint32_t sfw_smem = smem_base + ring.off_sfw(), sfx_smem = smem_base + ring.off_sfx();
+                    const uint32_t sf_cols = tmem_base + kSfCol0 + ring.stage * kSfColsPerStage;
                     const uint32_t tmem_sfw = sf_cols, tmem_sfx = sf_cols + 8;
-                    tcgen05_cp_32x128b_warpx4(tmem_sfw, make_sf_desc(sfw_smem + stage * L::kSfwBytes));
-                    tcgen05_cp_32x128b_warpx4(tmem_sfw + 4, make_sf_desc(sfw_smem + stage * L::kSfwBytes + 512));
-                    tcgen05_cp_32x128b_warpx4(tmem_sfx, make_sf_desc(sfx_smem + stage * L::kSfxBytes));
-                    if (n_tok > 128) tcgen05_cp_32x128b_warpx4(tmem_sfx + 4, make_sf_desc(sfx_smem + stage * L::kSfxBytes + 512));
-                    const uint64_t wdesc = make_kmajor_sw128_desc(w_base + stage * L::kWBytes);
-                    const uint64_t xdesc = make_kmajor_sw128_desc(x_base + stage * L::kXBytes);
+                    tcgen05_cp_32x128b_warpx4(tmem_sfw, make_sf_desc(sfw_smem));
+                    tcgen05_cp_32x128b_warpx4(tmem_sfw + 4, make_sf_desc(sfw_smem + 512));
+                    tcgen05_cp_32x128b_warpx4(tmem_sfx, make_sf_desc(sfx_smem));
+                    if (n_tok > 128) tcgen05_cp_32x128b_warpx4(tmem_sfx + 4, make_sf_desc(sfx_smem + 512));
+                    const uint64_t wdesc = make_kmajor_sw128_desc(smem_base + ring.off_w());
+                    const uint64_t xdesc = make_kmajor_sw128_desc(smem_base + ring.off_x());
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < 4; ++k4) {
                         const uint32_t id = idesc_with_sf_ids(idesc, k4, k4);
@@ -245,10 +300,10 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                         tcgen05_mma_mxf8f6f4(tmem_base + kAcc1Col, wdesc + (16384 >> 4) + k4 * 2, xdesc + k4 * 2, id, tmem_sfw + 4,
                                              tmem_sfx, acc);
                     }
-                    tcgen05_commit(empty_bar + stage);
+                    tcgen05_commit(empty_bar + ring.stage);
                     if (kb == num_kb - 1) tcgen05_commit(tmem_full_bar);
                 }
-                if (++stage == kStages) { stage = 0; phase ^= 1; }
+                ring.advance();
             }
         }
     }
@@ -301,6 +356,9 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 }
 #pragma unroll
                 for (int i = 0; i < kHalf; ++i) {
+                    // (leaving early, not stepping over the rest: the walk is unrolled over kHalf tokens, and skipping body after
+                    // body fetches all of that code; a tile of one token took 50 us of it)
+                    if (i % 4 == 0 && i >= my_tokens) break;
                     if (i < my_tokens) {
                         const float w = __shfl_sync(0xffffffffu, w_reg[i / 32], i % 32);
                         float gv = bf16_round(__uint_as_float(a0[i]));
@@ -326,6 +384,7 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.d) + t.w_block * 256 + channel;
 #pragma unroll
                 for (int i = 0; i < kHalf; ++i) {
+                    if (i % 4 == 0 && i >= my_tokens) break;
                     if (i < my_tokens) {
                         const long long row = static_cast<long long>(t.row_start) + col0 + i;
                         out[row * p.d_row_stride] = __float2bfloat16_rn(__uint_as_float(a0[i]));
