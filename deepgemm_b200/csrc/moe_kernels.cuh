@@ -153,7 +153,16 @@ dgb200_moe_gather_kernel(const unsigned char* __restrict__ x, const unsigned* __
         const int token = src / topk;
         const uint4* from = reinterpret_cast<const uint4*>(x + static_cast<long long>(token) * row_bytes);
         uint4* to = reinterpret_cast<uint4*>(acts + static_cast<long long>(row0 + r) * row_bytes);
-        for (int c = lane; c < row_bytes / 16; c += 32) to[c] = ld_global_nc_v4(from + c);
+        // seven loads in flight per lane
+        for (int c0 = lane; c0 < row_bytes / 16; c0 += 32 * 7) {
+            uint4 v[7];
+#pragma unroll
+            for (int j = 0; j < 7; ++j)
+                if (c0 + 32 * j < row_bytes / 16) v[j] = ld_global_nc_v4(from + c0 + 32 * j);
+#pragma unroll
+            for (int j = 0; j < 7; ++j)
+                if (c0 + 32 * j < row_bytes / 16) to[c0 + 32 * j] = v[j];
+        }
         for (int c = lane; c < sf_per_row; c += 32) sf_tile[c * 33 + r] = x_sf[static_cast<long long>(token) * sf_per_row + c];
     }
     __syncthreads();
@@ -221,6 +230,7 @@ struct PeerTable {
 // dest_row < 0 are skipped. One CTA per token; a thread owns 8 consecutive channels (one 16-byte vector per slot).
 // With shared experts their output row of the token (local, bf16 [tokens, hidden] at `shared_rows`) is one more slot,
 // added after the top-k slots (the reference gives it combine slot index num_topk, ...mega_moe.cuh:1275-1278).
+// Few tokens: the blocks of a grid column share a token's channels.
 // Reference: the combine of the fused kernel, deep_gemm/include/deep_gemm/impls/sm100_fp8_fp4_mega_moe.cuh:1323-1452.
 __global__ void __launch_bounds__(128)
 dgb200_moe_combine_kernel(const PeerTable peers, long long rows_offset, const long long* __restrict__ topk_idx,
@@ -242,17 +252,26 @@ dgb200_moe_combine_kernel(const PeerTable peers, long long rows_offset, const lo
         slot_rows[threadIdx.x] = addr;
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < hidden / 8; c += blockDim.x) {
+    // four slots' loads in flight before the first is added, in slot order (one after another, a 4-token combine took 17 us)
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < hidden / 8; c += gridDim.y * blockDim.x) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int k = 0; k <= topk; ++k) {
-            const unsigned long long addr = slot_rows[k];
-            if (addr == 0) continue;
-            const uint4 v = ld_global_nc_v4(reinterpret_cast<const uint4*>(addr) + c);
-            const unsigned w[4] = {v.x, v.y, v.z, v.w};
+        for (int k0 = 0; k0 <= topk; k0 += 4) {
+            unsigned long long addr[4];
+            uint4 v[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                acc[2 * i] += __uint_as_float(w[i] << 16);
-                acc[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+            for (int k = 0; k < 4; ++k) {
+                addr[k] = k0 + k <= topk ? slot_rows[k0 + k] : 0ull;
+                if (addr[k] != 0) v[k] = ld_global_nc_v4(reinterpret_cast<const uint4*>(addr[k]) + c);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (addr[k] == 0) continue;
+                const unsigned w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[2 * i] += __uint_as_float(w[i] << 16);
+                    acc[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+                }
             }
         }
         uint4 o;
@@ -932,7 +951,8 @@ dgb200_moe_combine_returned_kernel(const __nv_bfloat16* __restrict__ returned, c
 // dgb200_cast_rows_kernel<false>, i.e. per_token_cast_to_fp8(use_ue8m0=True, gran_k=32)) and writes row and packed
 // scales straight into each of its top-k destination rows of the expert-sorted buffers, on this rank or a peer.
 // `write_meta` also stores the routing weight and the source entry next to the row (the expert-parallel push does
-// that; on a single rank the plan kernels already have).
+// that; on a single rank the plan kernels already have). The blocks of a grid column share a token's row in steps
+// of 512 columns.
 __global__ void __launch_bounds__(256)
 dgb200_moe_quant_dispatch_kernel(const __nv_bfloat16* __restrict__ x, long long x_row_stride,
                                  const long long* __restrict__ topk_idx, const float* __restrict__ topk_weights,
@@ -955,36 +975,30 @@ dgb200_moe_quant_dispatch_kernel(const __nv_bfloat16* __restrict__ x, long long 
         if (d >= 0) {
             my_dest = d;
             my_base = peers.p[static_cast<int>(topk_idx[entry]) / experts_per_rank];
-            if (write_meta) {
+            if (write_meta && blockIdx.y == 0) {
                 reinterpret_cast<float*>(my_base + weight_offset)[d] = topk_weights[entry];
                 reinterpret_cast<int*>(my_base + src_offset)[d] = my_rank * entries_per_rank + entry;
             }
         }
     }
     const __nv_bfloat16* row = x + static_cast<long long>(token) * x_row_stride;
-    for (int col0 = 0; col0 < hidden; col0 += 512) {
+    for (int col0 = static_cast<int>(blockIdx.y) * 512; col0 < hidden; col0 += static_cast<int>(gridDim.y) * 512) {
         const int col = col0 + lane * 16;
         const bool valid = col < hidden;  // hidden is a multiple of 128
-        float v[16];
+        uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
         if (valid) {
             const uint4* src = reinterpret_cast<const uint4*>(row + col);
-            const uint4 r0 = ld_global_nc_v4(src), r1 = ld_global_nc_v4(src + 1);
-            const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[2 * i] = __uint_as_float(w[i] << 16);
-                v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+            r0 = ld_global_nc_v4(src);
+            r1 = ld_global_nc_v4(src + 1);
         }
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+        float v[16];
+        unpack_bf16x16(w, v);
+        bool special;
+        float amax = amax_bf16x16(w, special);
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));  // two lanes share a 32-element scale group
         const uint32_t e = ue8m0_ceil_bits(fmaxf(amax, 1e-4f) / 448.0f);
-        const float inv = 1.0f / __uint_as_float(e << 23);
+        const float inv = ue8m0_inverse(e);
         uint32_t o[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -1033,33 +1047,24 @@ dgb200_moe_quant_dispatch_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long
     const int my_dest = lane < topk ? dest_row[token * topk + lane] : -1;
     const float s_t = __ldg(tensor_scale);
     const __nv_bfloat16* row = x + static_cast<long long>(token) * x_row_stride;
-    for (int col0 = 0; col0 < hidden; col0 += 512) {
+    for (int col0 = static_cast<int>(blockIdx.y) * 512; col0 < hidden; col0 += static_cast<int>(gridDim.y) * 512) {
         const int col = col0 + lane * 16;  // one NVFP4 block per lane
         const bool valid = col < hidden;   // hidden is a multiple of 64
-        float v[16];
-        float amax = 0.0f;
+        uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
         if (valid) {
             const uint4* src = reinterpret_cast<const uint4*>(row + col);
-            const uint4 r0 = ld_global_nc_v4(src), r1 = ld_global_nc_v4(src + 1);
-            const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[2 * i] = __uint_as_float(w[i] << 16);
-                v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-                amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+            r0 = ld_global_nc_v4(src);
+            r1 = ld_global_nc_v4(src + 1);
         }
+        const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+        float v[16];
+        unpack_bf16x16(w, v);
+        bool special;
+        const float amax = amax_bf16x16(w, special);
         const uint32_t sf_byte = e4m3_byte(amax / 6.0f / s_t);
         const float factor = e4m3_to_float(sf_byte) * s_t;
-        uint32_t lo = 0, hi = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            lo |= (factor > 0.0f ? e2m1_code(v[i] / factor) : 0u) << (4 * i);
-            hi |= (factor > 0.0f ? e2m1_code(v[8 + i] / factor) : 0u) << (4 * i);
-        }
+        uint32_t lo, hi;
+        e2m1_codes_of_quotients(v, factor, special, lo, hi);
         // packed scale int of 64 elements = the scale bytes of lanes L .. L + 3 (L a multiple of 4)
         const uint32_t b1 = __shfl_down_sync(0xffffffffu, sf_byte, 1), b2 = __shfl_down_sync(0xffffffffu, sf_byte, 2),
                        b3 = __shfl_down_sync(0xffffffffu, sf_byte, 3);
