@@ -1,7 +1,6 @@
 """BF16 x BF16 GEMMs with the reference's Python signatures (csrc/apis/gemm.hpp:404-564, pybind defaults at
 :722-753): the same persistent tcgen05 kernel as the FP8 x FP4 family, issued as kind::f16 without scale factors.
 Outputs are written in place; nothing is returned."""
-import ctypes
 from typing import Optional
 
 import torch
@@ -12,7 +11,7 @@ from .runtime import get_mk_alignment_for_contiguous_layout
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _check_bf16(t: torch.Tensor, rank: int, name: str, allow_mn_major: bool = False):
@@ -55,7 +54,7 @@ def bf16_gemm_nt(a: torch.Tensor, b: torch.Tensor, d: torch.Tensor, c: Optional[
     accumulate = _prepare_accumulator(c, d)
     a_mn, a_stride = _b_major(a, 'a')
     b_mn, b_stride = _b_major(b, 'b')
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_bf16_gemm_nt(_p(a), a_stride, a_mn, _p(b), b_stride, b_mn, _p(d), d.stride(0), m, n, k,
                                                   int(d.dtype == torch.float32), accumulate, _lib.current_stream_ptr()))
 
@@ -105,7 +104,7 @@ def m_grouped_bf16_gemm_nt_contiguous(a: torch.Tensor, b: torch.Tensor, d: torch
             raise RuntimeError('expected_m_for_psum_layout is only valid with use_psum_layout')
     if m == 0:
         return
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_m_grouped_bf16_gemm_nt_contiguous(
             _p(a), a.stride(0), _p(b), b_stride, b_mn, _p(d), d.stride(0), _p(grouped_layout), m, n, k, num_groups, 0,
             1 if use_psum_layout else 0, get_mk_alignment_for_contiguous_layout(),
@@ -136,7 +135,7 @@ def m_grouped_bf16_gemm_nt_masked(a: torch.Tensor, b: torch.Tensor, d: torch.Ten
         raise RuntimeError('expected_m, m, n, k and num_groups must be positive')
     if masked_m.dtype != torch.int32 or not masked_m.is_contiguous() or not masked_m.is_cuda:
         raise RuntimeError('masked_m must be a contiguous CUDA int32 tensor')
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_m_grouped_bf16_gemm_nt_masked(
             _p(a), _p(b), _p(d), d.stride(1), _p(masked_m), num_groups, m, n, k, int(expected_m), 0,
             _lib.current_stream_ptr()))

@@ -1,6 +1,5 @@
 """m-grouped FP8 x FP4 (or FP8 x FP8) GEMMs with the reference's Python signatures
 (csrc/apis/gemm.hpp:166-297, pybind defaults at :673-694). Outputs are written in place; nothing is returned."""
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -13,7 +12,7 @@ kPackedFP4 = torch.int8  # two E2M1 codes per byte, logical K = 2 x last dim (re
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _check_ab(t: torch.Tensor, rank: int, name: str):
@@ -85,7 +84,7 @@ def fp8_fp4_gemm_nt(a: Tuple[torch.Tensor, torch.Tensor], b: Tuple[torch.Tensor,
     accumulate = _prepare_accumulator(c, d)
     sfa, sfb, gran_a, gran_b = transform_sf_pair_into_required_layout(
         a_sf, b_sf, m, n, k, recipe, recipe_a, recipe_b, None, None, disable_ue8m0_cast)
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_fp8_fp4_gemm_nt(
             _p(a_q), _p(sfa), sfa.stride(-1), _p(b_q), _p(sfb), sfb.stride(-1), _p(d), d.stride(0), m, n, k, gran_a, gran_b,
             int(b_q.dtype == kPackedFP4), int(d.dtype == torch.float32), accumulate, _lib.current_stream_ptr()))
@@ -138,7 +137,7 @@ def m_grouped_fp8_fp4_gemm_nt_contiguous(a: Tuple[torch.Tensor, torch.Tensor], b
         grouped_layout if use_psum_layout else None)
     entry = _lib.lib().dgb200_m_grouped_fp8_fp4_gemm_nn_contiguous if b_mn_major else \
         _lib.lib().dgb200_m_grouped_fp8_fp4_gemm_nt_contiguous
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(entry(
             _p(a_q), _p(sfa), sfa.stride(-1), _p(b_q), _p(sfb), sfb.stride(-1), sfb.stride(0),
             _p(d), d.stride(0), _p(grouped_layout), m, n, k, num_groups, gran_a, gran_b,
@@ -182,7 +181,7 @@ def m_grouped_fp8_fp4_gemm_nt_masked(a: Tuple[torch.Tensor, torch.Tensor], b: Tu
         raise RuntimeError('masked_m must be a contiguous CUDA int32 tensor')
     sfa, sfb, gran_a, gran_b = transform_sf_pair_into_required_layout(
         a_sf, b_sf, m, n, k, recipe, recipe_a, recipe_b, num_groups, num_groups, disable_ue8m0_cast)
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_m_grouped_fp8_fp4_gemm_nt_masked(
             _p(a_q), _p(sfa), sfa.stride(-1), sfa.stride(0), _p(b_q), _p(sfb), sfb.stride(-1), sfb.stride(0),
             _p(d), d.stride(1), _p(masked_m), num_groups, m, n, k, int(expected_m), gran_a, gran_b,

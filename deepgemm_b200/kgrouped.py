@@ -1,7 +1,6 @@
 """K-grouped GEMMs (MoE weight gradient) with the reference's Python signatures (k_grouped_fp8_gemm_tn_contiguous,
 csrc/apis/gemm.hpp:299-346, and k_grouped_bf16_gemm_tn_contiguous, :566-608; pybind defaults at :695-701 and :752-757).
 d is written in place."""
-import ctypes
 from typing import List, Optional, Tuple
 
 import torch
@@ -11,7 +10,7 @@ from .runtime import get_mk_alignment_for_contiguous_layout
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _check_ks(ks_cpu, num_groups, use_psum_layout, block_k, rows_of_a):
@@ -66,7 +65,7 @@ def k_grouped_fp8_gemm_tn_contiguous(a: Tuple[torch.Tensor, torch.Tensor], b: Tu
             raise RuntimeError(f'{name} must be a contiguous CUDA float8_e4m3fn [{sum_k}, {mn}] tensor')
         if sf.dtype != torch.float32 or tuple(sf.shape) != (sf_rows, mn) or not sf.is_contiguous():
             raise RuntimeError(f'scale factors of {name} must be contiguous float32 [{sf_rows}, {mn}]')
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         nbytes = _lib.lib().dgb200_k_grouped_sf_workspace_bytes(num_groups, m, n, sum_k)
         workspace = torch.empty(max(int(nbytes), 16), dtype=torch.int8, device=d.device)
         _lib.check(_lib.lib().dgb200_k_grouped_fp8_gemm_tn_contiguous(
@@ -93,7 +92,7 @@ def k_grouped_bf16_gemm_tn_contiguous(a: torch.Tensor, b: torch.Tensor, d: torch
     for t, mn, name in ((a, m, 'a'), (b, n, 'b')):
         if t.dtype != torch.bfloat16 or tuple(t.shape) != (sum_k, mn) or not t.is_contiguous() or not t.is_cuda:
             raise RuntimeError(f'{name} must be a contiguous CUDA bfloat16 [{sum_k}, {mn}] tensor')
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_k_grouped_bf16_gemm_tn_contiguous(
             _p(a), _p(b), _p(c), _p(d), _p(grouped_layout), int(use_psum_layout), get_mk_alignment_for_contiguous_layout(),
             num_groups, m, n, sum_k, _lib.current_stream_ptr()))

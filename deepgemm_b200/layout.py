@@ -1,10 +1,10 @@
 """Scale-factor layout transforms (reference: csrc/apis/layout.hpp:14-90, csrc/utils/layout.hpp:74-127)."""
-import ctypes
 from typing import Optional, Tuple, Union
 
 import torch
 
 from . import _lib
+from .runtime import get_mk_alignment_for_contiguous_layout
 from .utils.math import align, ceil_div
 
 
@@ -31,21 +31,22 @@ def check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups, tma_stride_check=Fal
         raise RuntimeError(f'scale factors must be {type_check}')
     if sf.dtype not in (torch.float32, torch.int32):
         raise RuntimeError('scale factors must be float32 or int32')
-    if sf.dim() != (3 if num_groups is not None else 2):
+    shape, per_elem = sf.shape, 1 if sf.dtype == torch.float32 else 4
+    if len(shape) != (3 if num_groups is not None else 2):
         raise RuntimeError('scale-factor rank does not match num_groups')
-    if num_groups is not None and sf.size(-3) != num_groups:
+    if num_groups is not None and shape[0] != num_groups:
         raise RuntimeError('scale-factor group count mismatch')
-    if sf.size(-2) != ceil_div(mn, gran_mn):
-        raise RuntimeError(f'scale-factor MN extent {sf.size(-2)} != ceil({mn} / {gran_mn})')
-    per_elem = 1 if sf.dtype == torch.float32 else 4
-    if sf.size(-1) != ceil_div(k, gran_k * per_elem):
-        raise RuntimeError(f'scale-factor K extent {sf.size(-1)} != ceil({k} / {gran_k * per_elem})')
+    if shape[-2] != ceil_div(mn, gran_mn):
+        raise RuntimeError(f'scale-factor MN extent {shape[-2]} != ceil({mn} / {gran_mn})')
+    if shape[-1] != ceil_div(k, gran_k * per_elem):
+        raise RuntimeError(f'scale-factor K extent {shape[-1]} != ceil({k} / {gran_k * per_elem})')
     if tma_stride_check:
-        if num_groups is not None and sf.stride(-3) != sf.stride(-1) * sf.size(-1):
+        stride = sf.stride()
+        if num_groups is not None and stride[0] != stride[-1] * shape[-1]:
             raise RuntimeError('packed scale factors: group stride must be K extent x K stride')
-        if not (sf.stride(-2) == 1 or mn == 1):
+        if not (stride[-2] == 1 or mn == 1):
             raise RuntimeError('packed scale factors must be MN-major')
-        if sf.stride(-1) != get_tma_aligned_size(mn, sf.element_size()):
+        if stride[-1] != get_tma_aligned_size(mn, 4):
             raise RuntimeError('packed scale factors: K stride must be the TMA-aligned MN size')
     return sf
 
@@ -56,22 +57,21 @@ def get_mn_major_tma_aligned_packed_ue8m0_tensor(sf: torch.Tensor, psum_layout: 
     Reference: csrc/jit_kernels/impls/smxx_layout.hpp:180-253."""
     if not (sf.is_cuda and sf.dtype == torch.float32 and sf.dim() in (2, 3)):
         raise RuntimeError('expected a 2-D or 3-D CUDA float32 tensor')
-    squeeze = sf.dim() == 2
-    sf3 = sf.unsqueeze(0) if squeeze else sf
-    g, mn, sf_k = sf3.shape
+    *lead, mn, sf_k = sf.shape
+    *lead_stride, stride_mn, stride_k = sf.stride()
+    g, stride_g = (lead[0], lead_stride[0]) if lead else (1, mn * stride_mn)
     packed_k, aligned_mn = ceil_div(sf_k, 4), align(mn, 4)
-    out = torch.empty((g, packed_k, aligned_mn), dtype=torch.int32, device=sf.device)
-    from .runtime import get_mk_alignment_for_contiguous_layout
-    with torch.cuda.device(sf.device):
+    # one allocation, made in the shape and strides it is returned in: rows beyond mn (up to a multiple of 4) are its tail
+    out = torch.empty_strided((*lead, aligned_mn, packed_k), ((packed_k * aligned_mn,) if lead else ()) + (1, aligned_mn),
+                              dtype=torch.int32, device=sf.device)
+    with _lib.on_device(sf.device):
         _lib.check(_lib.lib().dgb200_transform_sf_into_required_layout(
-            ctypes.c_void_p(sf3.data_ptr()), sf3.stride(0), sf3.stride(1), sf3.stride(2), ctypes.c_void_p(out.data_ptr()),
-            g, mn, sf_k, 1,
-            ctypes.c_void_p(psum_layout.data_ptr()) if psum_layout is not None else None,
+            sf.data_ptr(), stride_g, stride_mn, stride_k, out.data_ptr(), g, mn, sf_k, 1,
+            psum_layout.data_ptr() if psum_layout is not None else None,
             psum_layout.numel() if psum_layout is not None else 0,
             (psum_alignment or get_mk_alignment_for_contiguous_layout()) if psum_layout is not None else 0,
             _lib.current_stream_ptr()))
-    view = out.transpose(1, 2)[:, :mn, :]
-    return view[0] if squeeze else view
+    return out if aligned_mn == mn else out.narrow(-2, 0, mn)
 
 
 def transform_sf_into_required_layout(sf: torch.Tensor, mn: int, k: int,
@@ -81,6 +81,8 @@ def transform_sf_into_required_layout(sf: torch.Tensor, mn: int, k: int,
                                       psum_layout: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Reference: transform_sf_into_required_layout, csrc/apis/layout.hpp:14-61 (the sm_100 branches)."""
     gran_mn, gran_k = _recipe_grans(tuple(recipe), is_sfa)
+    if sf.dtype == torch.int32 and gran_mn == 1 and gran_k in (32, 128):
+        return check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups, tma_stride_check=True, type_check=torch.int32)
     check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups)
     if sf.dtype == torch.float32 and gran_k in (32, 128):
         if disable_ue8m0_cast:
@@ -89,8 +91,6 @@ def transform_sf_into_required_layout(sf: torch.Tensor, mn: int, k: int,
             index = torch.arange(mn, device=sf.device) // gran_mn
             sf = sf.index_select(-2, index)
         return get_mn_major_tma_aligned_packed_ue8m0_tensor(sf, psum_layout)
-    if sf.dtype == torch.int32 and gran_mn == 1 and gran_k in (32, 128):
-        return check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups, tma_stride_check=True, type_check=torch.int32)
     raise RuntimeError('Unknown SF transformation')
 
 

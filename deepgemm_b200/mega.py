@@ -315,7 +315,7 @@ def _run_layer(y, l1_weights, l2_weights, b, shared_l1_weights, shared_l2_weight
         peer_l1_w_sf=ctypes.cast(peer_w[1], ctypes.c_void_p) if spill is not None else None,
         peer_l2_w=ctypes.cast(peer_w[2], ctypes.c_void_p) if spill is not None else None,
         peer_l2_w_sf=ctypes.cast(peer_w[3], ctypes.c_void_p) if spill is not None else None)
-    with torch.cuda.device(y.device):
+    with _lib.on_device(y.device):
         _lib.check(_lib.lib().dgb200_fp8_fp4_mega_moe_ex(ctypes.byref(args), _lib.current_stream_ptr()))
 
 
@@ -381,8 +381,8 @@ def nvfp4_mega_moe(y: torch.Tensor, l1_weights: Tuple[torch.Tensor, torch.Tensor
     if stats is not None and not (stats.dtype == torch.int32 and stats.numel() == num_local and stats.is_contiguous()):
         raise RuntimeError('cumulative_local_expert_recv_stats must be a contiguous int32 [num_local_experts] tensor')
     ptrs = (ctypes.c_uint64 * len(b.handle.buffer_ptrs))(*[int(p) for p in b.handle.buffer_ptrs])
-    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
-    with torch.cuda.device(y.device):
+    p = lambda t: t.data_ptr() if t is not None else None
+    with _lib.on_device(y.device):
         _lib.check(_lib.lib().dgb200_nvfp4_mega_moe(
             p(y), p(l1_weights[0]), p(l1_weights[1]), p(l1_weights[2]), p(l2_weights[0]), p(l2_weights[1]),
             p(l2_weights[2]), p(x_scale), p(act_scale), p(stats), p(b.buffer), ctypes.cast(ptrs, ctypes.c_void_p),
@@ -419,8 +419,8 @@ def nvfp4_mega_moe_bf16_input(y: torch.Tensor, x: torch.Tensor, l1_weights: Tupl
     stats = cumulative_local_expert_recv_stats
     if stats is not None and not (stats.dtype == torch.int32 and stats.numel() == b.num_experts and stats.is_contiguous()):
         raise RuntimeError('cumulative_local_expert_recv_stats must be a contiguous int32 [num_experts] tensor')
-    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
-    with torch.cuda.device(y.device):
+    p = lambda t: t.data_ptr() if t is not None else None
+    with _lib.on_device(y.device):
         _lib.check(_lib.lib().dgb200_nvfp4_mega_moe_bf16_input(
             p(y), p(x), x.stride(0), p(logits), p(l1_weights[0]), p(l1_weights[1]), p(l1_weights[2]), p(l2_weights[0]),
             p(l2_weights[1]), p(l2_weights[2]), p(x_scale), p(act_scale), p(stats), p(b.buffer), y.size(0),
@@ -464,8 +464,8 @@ def bf16_mega_moe(y: torch.Tensor, l1_weights: torch.Tensor, l2_weights: torch.T
     if stats is not None and not (stats.dtype == torch.int32 and stats.numel() == num_local and stats.is_contiguous()):
         raise RuntimeError('cumulative_local_expert_recv_stats must be a contiguous int32 [num_local_experts] tensor')
     ptrs = (ctypes.c_uint64 * len(b.handle.buffer_ptrs))(*[int(p) for p in b.handle.buffer_ptrs])
-    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
-    with torch.cuda.device(y.device):
+    p = lambda t: t.data_ptr() if t is not None else None
+    with _lib.on_device(y.device):
         _lib.check(_lib.lib().dgb200_bf16_mega_moe(
             p(y), p(l1_weights), p(l2_weights), p(shared_l1_weights), p(shared_l2_weights), shared_inter, p(stats), p(b.buffer),
             ctypes.cast(ptrs, ctypes.c_void_p), b.rank,
@@ -486,7 +486,7 @@ def route_sigmoid_topk(logits: torch.Tensor, num_topk: int, topk_idx: Optional[t
     if topk_weights is None:
         topk_weights = torch.empty((t, num_topk), dtype=torch.float32, device=logits.device)
     assert topk_idx.is_contiguous() and topk_weights.is_contiguous()
-    with torch.cuda.device(logits.device):
+    with _lib.on_device(logits.device):
         _lib.check(_lib.lib().dgb200_route_sigmoid_topk(
             ctypes.c_void_p(logits.data_ptr()), t, e, num_topk, ctypes.c_void_p(topk_idx.data_ptr()),
             ctypes.c_void_p(topk_weights.data_ptr()), _lib.current_stream_ptr()))

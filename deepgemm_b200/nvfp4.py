@@ -5,7 +5,6 @@ follow its conventions for the FP8 x FP4 path (tuples of (values, scales), outpu
 ``use_psum_layout``), with the per-tensor scale added as a third tuple element. Everything runs in libdgb200.so
 (tcgen05 ``kind::mxf4nvf4`` with ``scale_vec::4X``); there is no fallback.
 """
-import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -16,7 +15,7 @@ from .utils.math import align
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _check_x(x: torch.Tensor) -> torch.Tensor:
@@ -31,7 +30,7 @@ def nvfp4_tensor_scale(x: torch.Tensor) -> torch.Tensor:
     """FP32 scalar amax(|x|) / (6 * 448) (1.0 for an all-zero tensor), on the device."""
     x = _check_x(x)
     out = torch.empty((), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().dgb200_nvfp4_tensor_scale(_p(x), x.stride(0), x.size(0), x.size(1), _p(out),
                                                         _lib.current_stream_ptr()))
     return out
@@ -59,7 +58,7 @@ def per_token_cast_to_nvfp4(x: torch.Tensor, tensor_scale: Optional[torch.Tensor
         k_stride, row_stride = align(m, 4), 1
     else:
         raise RuntimeError(f'unknown sf_layout `{sf_layout}`')
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().dgb200_per_token_cast_to_nvfp4(_p(x), x.stride(0), m, k, _p(tensor_scale), _p(q), q.stride(0),
                                                              _p(packed), k_stride, row_stride, _lib.current_stream_ptr()))
     sf = packed.view(torch.uint8).view(torch.float8_e4m3fn) if sf_layout == 'token' else packed
@@ -77,7 +76,7 @@ def per_token_cast_to_nvfp4_into(x: torch.Tensor, tensor_scale: torch.Tensor, q_
     if not (sf_packed_out.dtype == torch.int32 and sf_packed_out.shape[0] >= m and sf_packed_out.shape[1] == k // 64 and
             sf_packed_out.stride(1) == 1):
         raise RuntimeError('sf_packed_out must be int32 [>= M, K / 64], token-major')
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().dgb200_per_token_cast_to_nvfp4(_p(x), x.stride(0), m, k, _p(tensor_scale), _p(q_out),
                                                              q_out.stride(0), _p(sf_packed_out), 1, sf_packed_out.stride(0),
                                                              _lib.current_stream_ptr()))
@@ -141,7 +140,7 @@ def m_grouped_nvfp4_gemm_nt_contiguous(a: Tuple[torch.Tensor, torch.Tensor, torc
         return
     sfa = _sf_mn_major(a_sf, m, k, (), 'a')
     sfb = _sf_mn_major(b_sf, n, k, (num_groups,), 'b')
-    with torch.cuda.device(d.device):
+    with _lib.on_device(d.device):
         _lib.check(_lib.lib().dgb200_m_grouped_nvfp4_gemm_nt_contiguous(
             _p(a_q), _p(sfa), sfa.stride(-1), _p(a_scale), _p(b_q), _p(sfb), sfb.stride(-1), sfb.stride(0) if num_groups > 1 else
             sfb.stride(-1) * sfb.size(-1), _p(b_scales), _p(d), d.stride(0), _p(grouped_layout), m, n, k, num_groups,

@@ -4,7 +4,6 @@ The quantisers run as CUDA kernels of libdgb200.so (fused amax / UE8M0 scale / c
 tensors. The dequantisers and the packing helpers are plain tensor expressions: the reference uses them only to
 build test inputs and expected values, and they work on any device.
 """
-import ctypes
 from typing import Tuple
 
 import torch
@@ -21,7 +20,7 @@ def align(x: int, y: int) -> int:
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def ceil_to_ue8m0(x: torch.Tensor) -> torch.Tensor:
@@ -66,7 +65,7 @@ def _cast(x: torch.Tensor, gran_k: int, fp4: bool, want_f32: bool, packed_layout
         packed = torch.empty((packed_k, align(m, 4)), dtype=torch.int32, device=x.device).t()[:m]
         k_stride, row_stride = align(m, 4), 1
     fn = _lib.lib().dgb200_per_token_cast_to_fp4 if fp4 else _lib.lib().dgb200_per_token_cast_to_fp8
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(fn(_ptr(x), x.stride(0), m, k, gran_k, _ptr(q), q.stride(0), _ptr(sf), _ptr(packed), k_stride, row_stride,
                       _lib.current_stream_ptr()))
     return q, sf, packed
@@ -95,7 +94,7 @@ def per_channel_cast_to_fp8(x: torch.Tensor, use_ue8m0: bool, gran_k: int = 128)
         raise RuntimeError(f'K ({k}) must be a multiple of gran_k ({gran_k})')
     q = torch.empty((k, mn), dtype=torch.float8_e4m3fn, device=x.device)
     sf = torch.empty((k // gran_k, mn), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().dgb200_per_channel_cast_to_fp8(_ptr(x), k, mn, gran_k, _ptr(q), _ptr(sf), _lib.current_stream_ptr()))
     return q, sf
 
@@ -159,7 +158,7 @@ def per_token_cast_to_fp8_into(x: torch.Tensor, q_out: torch.Tensor, sf_packed_o
     if not (sf_packed_out.dtype == torch.int32 and sf_packed_out.shape[0] >= m and sf_packed_out.shape[1] == packed_k and
             sf_packed_out.stride(1) == 1):
         raise RuntimeError('sf_packed_out must be int32 [>= M, ceil(K / gran_k / 4)], token-major')
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         _lib.check(_lib.lib().dgb200_per_token_cast_to_fp8(
             _ptr(x), x.stride(0), m, k, gran_k, _ptr(q_out), q_out.stride(0), None, _ptr(sf_packed_out), 1,
             sf_packed_out.stride(0), _lib.current_stream_ptr()))
