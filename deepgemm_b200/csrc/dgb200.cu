@@ -556,10 +556,10 @@ int allow_row_mover_smem(Kernel kernel) {
 // The layer GEMMs with swapped operands (gemm_swap_kernel.cuh): weights on M, an expert's tokens on N. Takes the same
 // call description as run_gemm; only the FP8 x FP4 / FP8 x FP8 kind, the psum layout with 128-row segments, scale
 // factors in tcgen05.cp order and the SwiGLU / BF16 epilogues.
-template <int EPI, int kSmallTok>
+template <int EPI, int kSmallTok, bool kPlainSf = false>
 int launch_gemm_swap(const CUtensorMap& tm_x, const CUtensorMap& tm_xs, const CUtensorMap& tm_w, const CUtensorMap& tm_sfx,
                      const CUtensorMap& tm_sfxs, const CUtensorMap& tm_sfw, const GemmParams& p, int grid, cudaStream_t stream) {
-    auto kernel = dgb200_swap_gemm_kernel<EPI, kSmallTok>;
+    auto kernel = dgb200_swap_gemm_kernel<EPI, kSmallTok, kPlainSf>;
     constexpr int kBytes = SwapSmem<kSmallTok>::kDynamicBytes;
     static bool configured = false;
     static int configured_device = -1;
@@ -577,17 +577,25 @@ int launch_gemm_swap(const CUtensorMap& tm_x, const CUtensorMap& tm_xs, const CU
 
 int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     GemmParams& p = c.p;
-    DGB_REQUIRE(c.kind == kKindFp8Fp4 && p.mode == kModePsum && p.alignment == 128 && p.sf_transposed == 1,
-                "the swapped-operand kernel serves the FP8 layer path only");
-    DGB_REQUIRE(c.epilogue == kEpiSwiGLU || c.epilogue == kEpiBF16, "unknown epilogue %d for the swapped-operand kernel", c.epilogue);
+    const bool plain = p.mode == kModeMasked;  // the public masked GEMM: scale factors in plain row order
+    DGB_REQUIRE(c.kind == kKindFp8Fp4 && ((p.mode == kModePsum && p.alignment == 128 && p.sf_transposed == 1) || (plain && p.sf_transposed == 0)),
+                "the swapped-operand kernel serves the FP8 layer path and the masked GEMM");
+    DGB_REQUIRE(c.epilogue == kEpiBF16 || (c.epilogue == kEpiSwiGLU && !plain), "unknown epilogue %d for the swapped-operand kernel", c.epilogue);
     DGB_REQUIRE(p.k > 0 && p.k % 128 == 0 && p.n > 0 && p.n % 256 == 0, "k must be a multiple of 128 and n of 256");
     DGB_REQUIRE(p.num_groups > 0 && p.num_groups <= kMaxCachedGroups, "at most %d groups", kMaxCachedGroups);
-    DGB_REQUIRE(p.gran_a == 32 && p.gran_b == 32, "per-32 scales only");
-    DGB_REQUIRE(c.sfa_k_stride % 4 == 0 && c.sfb_k_stride % 4 == 0 && c.sfb_k_stride >= p.n && c.sfa_k_stride >= c.a_rows_total,
+    DGB_REQUIRE(p.gran_a == 32 || (plain && p.gran_a == 128), "gran_k_a must be 32 (or 128), got %d", p.gran_a);
+    DGB_REQUIRE(p.gran_b == 32 || (plain && p.gran_b == 128), "gran_k_b must be 32 (or 128), got %d", p.gran_b);
+    DGB_REQUIRE(reinterpret_cast<uintptr_t>(c.a) % 16 == 0 && reinterpret_cast<uintptr_t>(c.b) % 32 == 0 &&
+                    reinterpret_cast<uintptr_t>(c.sfa) % 16 == 0 && reinterpret_cast<uintptr_t>(c.sfb) % 16 == 0,
+                "a and the scale factors must be 16-byte aligned, b 32-byte");
+    DGB_REQUIRE(c.sfa_k_stride % 4 == 0 && c.sfb_k_stride % 4 == 0 && c.sfb_k_stride >= p.n && c.sfa_k_stride >= (plain ? p.m : c.a_rows_total),
                 "packed scale-factor strides must be multiples of 4 ints that cover MN");
-    const int packed_k = p.k / 128;
+    const int packed_k_a = (p.k / p.gran_a + 3) / 4, packed_k = (p.k / p.gran_b + 3) / 4;
+    DGB_REQUIRE(c.num_groups_a == 1 || c.sfa_group_stride == static_cast<long long>(packed_k_a) * c.sfa_k_stride,
+                "scale factors of A: group stride must equal packed K x MN stride");
     DGB_REQUIRE(p.num_groups == 1 || c.sfb_group_stride == static_cast<long long>(packed_k) * c.sfb_k_stride,
                 "scale factors of B: group stride must equal packed K x MN stride");
+    p.sfa_group_rows = c.num_groups_a > 1 ? packed_k_a : 0;
     p.sfb_packed_k = packed_k;
     if (c.a_rows_total == 0) return 0;
     CUtensorMap tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw;
@@ -598,10 +606,11 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     for (int i = 0; i < 2; ++i) {
         rc = make_tensor_map_2d(i == 0 ? &tm_x : &tm_xs, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.a, static_cast<uint64_t>(p.k),
                                 static_cast<uint64_t>(c.a_rows_total), static_cast<uint64_t>(p.k), 128,
-                                i == 0 ? kSwapMaxTok : (tiny ? 16 : 64), CU_TENSOR_MAP_SWIZZLE_128B);
+                                i == 0 ? kSwapMaxTok : (tiny ? 16 : 80), CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
         rc = make_tensor_map_2d(i == 0 ? &tm_sfx : &tm_sfxs, CU_TENSOR_MAP_DATA_TYPE_INT32, c.sfa, static_cast<uint64_t>(c.sfa_k_stride),
-                                static_cast<uint64_t>(packed_k), static_cast<uint64_t>(c.sfa_k_stride) * 4, i == 0 ? 256 : 128, 1,
+                                static_cast<uint64_t>(packed_k_a) * c.num_groups_a, static_cast<uint64_t>(c.sfa_k_stride) * 4,
+                                i == 0 ? 256 : 128, 1,
                                 CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc) return rc;
     }
@@ -625,11 +634,14 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     int sms = 0;
     rc = effective_num_sms(&sms);
     if (rc) return rc;
+    if (plain)
+        return tiny ? launch_gemm_swap<kEpiBF16, 16, true>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream)
+                    : launch_gemm_swap<kEpiBF16, 80, true>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
     if (c.epilogue == kEpiSwiGLU)
         return tiny ? launch_gemm_swap<kEpiSwiGLU, 16>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream)
-                    : launch_gemm_swap<kEpiSwiGLU, 64>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
+                    : launch_gemm_swap<kEpiSwiGLU, 80>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
     return tiny ? launch_gemm_swap<kEpiBF16, 16>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream)
-                : launch_gemm_swap<kEpiBF16, 64>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
+                : launch_gemm_swap<kEpiBF16, 80>(tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw, p, sms, stream);
 }
 
 // --------------------------------------------------------------------------------------------------------------
@@ -1870,6 +1882,12 @@ int dgb200_m_grouped_fp8_fp4_gemm_nt_masked(
     p.store_padding = 0;
     c.max_tiles = 0;
     c.expected_rows = std::min(expected_m, max_m);
+    // Few rows per group: tokens on the N side, so that the MMAs follow the row count and a group of up to 160 rows is one pass
+    // over its weights. Tokens on M -> swapped, 32 groups, N 4096, K 7168 (us): FP8 x FP4 8 rows 130 -> 113, 64 rows 140 -> 132,
+    // 128 rows 206 -> 159, 160 rows 230 -> 234; FP8 x FP8 170 -> 157, 185 -> 177, 256 -> 213, 288 -> 297.
+    if (!d_is_fp32 && n % 256 == 0 && num_groups <= kMaxCachedGroups && tuning().block_n == 0 && tuning().pair != 1 &&
+        (tuning().swap_ab == 1 || (tuning().swap_ab == -1 && expected_m > 0 && expected_m <= 128)))
+        return run_gemm_swap(c, static_cast<cudaStream_t>(stream));
     return run_gemm(c, static_cast<cudaStream_t>(stream));
 }
 

@@ -10,8 +10,10 @@
 //
 //   D^T[256 channels, tokens] = W[256, K] . X[tokens, K]^T     FP8 (E4M3) tokens x MXFP4 (E2M1) weights, UE8M0 per 32
 //
-// Layer path only: psum layout with 128-row expert segments, scale factors of both operands in tcgen05.cp row order,
+// Layer path: psum layout with 128-row expert segments, scale factors of both operands in tcgen05.cp row order,
 // gate/up rows interleaved by 128 (accumulator 0 = 128 gate channels, accumulator 1 = the matching up channels).
+// kPlainSf: the public masked GEMM with few rows per group; scale factors in plain row order, per 32 or per 128 K, transposed by the
+// otherwise idle warp 2 as in gemm_kernel.cuh.
 // An epilogue thread owns one channel (TMEM lane) and walks the tokens (TMEM columns):
 //   SwiGLU: bf16(gate), bf16(up) -> clamp -> silu(gate) * up * weight[token] -> amax over the warp's 32 channels (one
 //           UE8M0 scale group) -> e4m3; a warp writes the 32 bytes of one token's scale group at a time.
@@ -33,17 +35,17 @@ constexpr int kSwapMaxTok = 160;  // tokens per tile = largest UMMA N used (mult
 // last stages of the old layout have been consumed.
 template <int kSmallTok>
 struct SwapSmem {
-    static_assert(kSmallTok == 16 || kSmallTok == 64, "token slots of the small layout");
+    static_assert(kSmallTok == 16 || kSmallTok == 80, "token slots of the small layout");
     static constexpr int kSmallStages = kSmallTok == 16 ? 6 : 5, kLargeStages = 4;
     static constexpr int kStages = kSmallStages;       // barriers
     static constexpr int kWBytes = 256 * 128;          // 256 weight rows x 128 K bytes (packed FP4 expanded by TMA)
     static constexpr int kSfwBytes = 2 * 512;          // one packed scale int per weight row
     static constexpr int kSmallX = kSmallTok * 128, kLargeX = kSwapMaxTok * 128;  // token rows x 128 K bytes
     static constexpr int kSmallSfx = 512, kLargeSfx = 2 * 512;  // packed scale ints of 128 or 256 token rows
-    static constexpr int kRing = kLargeStages * (kWBytes + kLargeX + kSfwBytes + kLargeSfx);
-    static_assert(kSmallStages * (kWBytes + kSmallX + kSfwBytes + kSmallSfx) <= kRing, "both layouts share the ring");
-    static constexpr int kOffBar = kRing;
-    static constexpr int kNumBars = 2 * kStages + 2;
+    static constexpr int kSmallRing = kSmallStages * (kWBytes + kSmallX + kSfwBytes + kSmallSfx);
+    static constexpr int kLargeRing = kLargeStages * (kWBytes + kLargeX + kSfwBytes + kLargeSfx);
+    static constexpr int kOffBar = kSmallRing > kLargeRing ? kSmallRing : kLargeRing;  // both layouts share the ring
+    static constexpr int kNumBars = 3 * kStages + 2;
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;
     static constexpr int kOffGroups = kOffMisc + 16;
     static constexpr int kTotal = kOffGroups + 3 * kMaxCachedGroups * 4;
@@ -90,7 +92,8 @@ struct SwapRing {
 struct SwapTile {
     int group;      // expert
     int w_block;    // 256-row block of the expert's weight matrix
-    int row_start;  // first token row of the tile in the expert-sorted buffers (a multiple of 128)
+    int row_start;  // first token row of the tile in the expert-sorted buffers (a multiple of 128) or the flattened masked ones
+    int sf_row;     // first row of the tile in the scale factors: the same, or the row within the group (masked)
     int tokens;     // valid token rows of the tile (1 .. kSwapMaxTok)
 };
 
@@ -105,10 +108,11 @@ struct SwapScheduler {
     const int* start;      // first row of each group
     const int* tiles_end;  // running tile count
     int num_groups, num_w_blocks;
+    bool masked;
     int tile, g;
 
-    __device__ SwapScheduler(const int* lay_, const int* start_, const int* tiles_end_, int num_groups_, int num_w_blocks_)
-        : lay(lay_), start(start_), tiles_end(tiles_end_), num_groups(num_groups_), num_w_blocks(num_w_blocks_),
+    __device__ SwapScheduler(const int* lay_, const int* start_, const int* tiles_end_, const GemmParams& p)
+        : lay(lay_), start(start_), tiles_end(tiles_end_), num_groups(p.num_groups), num_w_blocks(p.n / 256), masked(p.mode == kModeMasked),
           tile(static_cast<int>(blockIdx.x)), g(0) {}
 
     __device__ bool next(SwapTile& t) {
@@ -121,6 +125,7 @@ struct SwapScheduler {
         t.group = g;
         t.w_block = local;
         t.row_start = start[g] + tt * 128;
+        t.sf_row = masked ? tt * 128 : t.row_start;
         t.tokens = rows <= kSwapMaxTok ? rows : min(128, rows - tt * 128);
         tile += static_cast<int>(gridDim.x);
         return true;
@@ -129,7 +134,7 @@ struct SwapScheduler {
 
 // tm_x / tm_xs: tokens [rows, K] bytes, box 128 x kSwapMaxTok / kSmallTok; tm_w: weights (16U4_ALIGN16B) box 128 x 256;
 // tm_sfx / tm_sfxs: packed scale ints of the tokens, box 256 / 128 x 1; tm_sfw: of the weights, box 256 x 1. p: the GemmParams of the layer call (psum layout, alignment 128).
-template <int EPI, int kSmallTok>
+template <int EPI, int kSmallTok, bool kPlainSf = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_xs,
                         const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_sfx,
@@ -151,6 +156,7 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     uint64_t* empty_bar = bars + kStages;
     uint64_t* tmem_full_bar = bars + 2 * kStages;
     uint64_t* tmem_empty_bar = bars + 2 * kStages + 1;
+    uint64_t* sf_ready_bar = bars + 2 * kStages + 2;  // kPlainSf: the transposer has turned the stage's scale factors
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 4);
 
@@ -163,6 +169,7 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         for (int i = 0; i < kStages; ++i) {
             mbar_init(full_bar + i, 2);   // token loader and weight loader
             mbar_init(empty_bar + i, 1);  // tcgen05.commit of the MMA issuer
+            if constexpr (kPlainSf) mbar_init(sf_ready_bar + i, 1);
         }
         mbar_init(tmem_full_bar, 1);
         mbar_init(tmem_empty_bar, 8);     // lane 0 of each epilogue warp
@@ -180,9 +187,15 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     int* group_start = group_lay + kMaxCachedGroups;
     int* group_tiles_end = group_start + kMaxCachedGroups;
     for (int i = threadIdx.x; i < p.num_groups; i += kGemmThreads) {
-        const int prev_end = i == 0 ? 0 : __ldg(p.layout + i - 1);
-        const int start = (prev_end + 127) / 128 * 128;
-        const int end = __ldg(p.layout + i);
+        int start, end;
+        if (p.mode == kModeMasked) {
+            start = i * p.m;
+            end = start + max(min(__ldg(p.layout + i), p.m), 0);
+        } else {
+            const int prev_end = i == 0 ? 0 : __ldg(p.layout + i - 1);
+            start = (prev_end + 127) / 128 * 128;
+            end = __ldg(p.layout + i);
+        }
         group_lay[i] = end;
         group_start[i] = start;
         group_tiles_end[i] = (group_selected(p, end - start) && group_in_range(p, i)) ? swap_token_tiles(end - start) * num_w_blocks : 0;
@@ -211,12 +224,14 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
     const int num_kb = p.k / 128;
+    // K blocks that one packed scale int covers
+    const int x_per = kPlainSf && p.gran_a == 128 ? 4 : 1, w_per = kPlainSf && p.gran_b == 128 ? 4 : 1;
 
     if (warp < 4) {
     setmaxnreg_dec<kRegsControlWarps>();
     if (warp == 0) {
         // ---------------------------------------------------------------- loader: token rows + their scale ints
-        SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
+        SwapScheduler sched(group_lay, group_start, group_tiles_end, p);
         SwapTile t;
         SwapRing<kSmallTok> ring;
         const bool leader = elect_one();
@@ -230,16 +245,17 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 if (!ok) break;
                 if (leader) {
                     uint64_t* bar = full_bar + ring.stage;
-                    mbar_arrive_expect_tx(bar, ring.x_bytes() + ring.sfx_bytes());
+                    const bool with_sf = kb % x_per == 0;
+                    mbar_arrive_expect_tx(bar, ring.x_bytes() + (with_sf ? ring.sfx_bytes() : 0));
                     tma_load_2d(smem + ring.off_x(), x_map, bar, kb * 128, t.row_start);
-                    tma_load_2d(smem + ring.off_sfx(), sfx_map, bar, t.row_start, kb);
+                    if (with_sf) tma_load_2d(smem + ring.off_sfx(), sfx_map, bar, t.sf_row, t.group * p.sfa_group_rows + kb / x_per);
                 }
                 ring.advance();
             }
         }
     } else if (warp == 3) {
         // ---------------------------------------------------------------- loader: weight rows + their scale ints
-        SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
+        SwapScheduler sched(group_lay, group_start, group_tiles_end, p);
         SwapTile t;
         SwapRing<kSmallTok> ring;
         const bool leader = elect_one();
@@ -253,16 +269,17 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 if (!ok) break;
                 if (leader) {
                     uint64_t* bar = full_bar + ring.stage;
-                    mbar_arrive_expect_tx(bar, p.b_tx_bytes + L::kSfwBytes);
+                    const bool with_sf = kb % w_per == 0;
+                    mbar_arrive_expect_tx(bar, p.b_tx_bytes + (with_sf ? L::kSfwBytes : 0));
                     tma_load_2d(smem + ring.off_w(), &tm_w, bar, kb * 128, w_row);
-                    tma_load_2d(smem + ring.off_sfw(), &tm_sfw, bar, t.w_block * 256, sfw_y + kb);
+                    if (with_sf) tma_load_2d(smem + ring.off_sfw(), &tm_sfw, bar, t.w_block * 256, sfw_y + kb / w_per);
                 }
                 ring.advance();
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
+        SwapScheduler sched(group_lay, group_start, group_tiles_end, p);
         SwapTile t;
         uint32_t iter = 0;
         SwapRing<kSmallTok> ring;
@@ -278,22 +295,28 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             const uint32_t n_tok = static_cast<uint32_t>((t.tokens + 15) & ~15);
             // weights are the A operand (E2M1 in byte containers or E4M3), tokens the B operand (E4M3)
             const uint32_t idesc = make_idesc_block_scaled(p.b_fmt, kFmtE4M3, 128, n_tok, kScaleUE8M0);
+            uint32_t tmem_sfw = 0, tmem_sfx = 0;  // TMEM columns holding the scale factors of the current K block
             for (int kb = 0; kb < num_kb; ++kb) {
-                ok = mbar_wait(full_bar + ring.stage, ring.phase(), abort_flag, kTimeoutFull, kb);
+                ok = mbar_wait((kPlainSf ? sf_ready_bar : full_bar) + ring.stage, ring.phase(), abort_flag, kTimeoutFull, kb);
                 if (!ok) break;
                 if (leader) {
                     const uint32_t sfw_smem = smem_base + ring.off_sfw(), sfx_smem = smem_base + ring.off_sfx();
                     const uint32_t sf_cols = tmem_base + kSfCol0 + ring.stage * kSfColsPerStage;
-                    const uint32_t tmem_sfw = sf_cols, tmem_sfx = sf_cols + 8;
-                    tcgen05_cp_32x128b_warpx4(tmem_sfw, make_sf_desc(sfw_smem));
-                    tcgen05_cp_32x128b_warpx4(tmem_sfw + 4, make_sf_desc(sfw_smem + 512));
-                    tcgen05_cp_32x128b_warpx4(tmem_sfx, make_sf_desc(sfx_smem));
-                    if (n_tok > 128) tcgen05_cp_32x128b_warpx4(tmem_sfx + 4, make_sf_desc(sfx_smem + 512));
+                    if (kb % w_per == 0) {
+                        tmem_sfw = sf_cols;
+                        tcgen05_cp_32x128b_warpx4(tmem_sfw, make_sf_desc(sfw_smem));
+                        tcgen05_cp_32x128b_warpx4(tmem_sfw + 4, make_sf_desc(sfw_smem + 512));
+                    }
+                    if (kb % x_per == 0) {
+                        tmem_sfx = sf_cols + 8;
+                        tcgen05_cp_32x128b_warpx4(tmem_sfx, make_sf_desc(sfx_smem));
+                        if (n_tok > 128) tcgen05_cp_32x128b_warpx4(tmem_sfx + 4, make_sf_desc(sfx_smem + 512));
+                    }
                     const uint64_t wdesc = make_kmajor_sw128_desc(smem_base + ring.off_w());
                     const uint64_t xdesc = make_kmajor_sw128_desc(smem_base + ring.off_x());
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < 4; ++k4) {
-                        const uint32_t id = idesc_with_sf_ids(idesc, k4, k4);
+                        const uint32_t id = idesc_with_sf_ids(idesc, w_per == 1 ? k4 : kb % 4, x_per == 1 ? k4 : kb % 4);
                         const uint32_t acc = (kb | k4) != 0 ? 1u : 0u;
                         // rows 0..127 of the weight tile -> accumulator 0, rows 128..255 (16 KB further) -> accumulator 1
                         tcgen05_mma_mxf8f6f4(tmem_base, wdesc + k4 * 2, xdesc + k4 * 2, id, tmem_sfw, tmem_sfx, acc);
@@ -306,6 +329,41 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 ring.advance();
             }
         }
+    } else if (kPlainSf && warp == 2) {
+        // ---------------------------------------------------------------- scale-factor transposer (see gemm_kernel.cuh)
+        SwapScheduler sched(group_lay, group_start, group_tiles_end, p);
+        SwapTile t;
+        SwapRing<kSmallTok> ring;
+        bool ok = true;
+        while (ok && sched.next(t)) {
+            (void)ring.enter(t.tokens);
+            const bool wide = t.tokens > 128;  // the tokens' scale factors fill a second block of 128
+            for (int kb = 0; kb < num_kb; ++kb) {
+                ok = mbar_wait(full_bar + ring.stage, ring.phase(), abort_flag, kTimeoutFull, kb);
+                if (!ok) break;
+                const bool do_w = kb % w_per == 0, do_x = kb % x_per == 0;
+                uint32_t* sw = reinterpret_cast<uint32_t*>(smem + ring.off_sfw());
+                uint32_t* sx = reinterpret_cast<uint32_t*>(smem + ring.off_sfx());
+                uint32_t vw[2][4], vx[2][4];
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (do_w) vw[b][j] = sw[b * 128 + j * 32 + lane];
+                        if (do_x && (b == 0 || wide)) vx[b][j] = sx[b * 128 + j * 32 + lane];
+                    }
+                __syncwarp();
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    if (do_w) *reinterpret_cast<uint4*>(sw + b * 128 + lane * 4) = make_uint4(vw[b][0], vw[b][1], vw[b][2], vw[b][3]);
+                    if (do_x && (b == 0 || wide)) *reinterpret_cast<uint4*>(sx + b * 128 + lane * 4) = make_uint4(vx[b][0], vx[b][1], vx[b][2], vx[b][3]);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sf_ready_bar + ring.stage);
+                ring.advance();
+            }
+        }
     }
     } else {
         setmaxnreg_inc<kRegsEpilogueWarps>();
@@ -314,7 +372,7 @@ dgb200_swap_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         // split the token columns in halves. Everything is drained to registers first so that the MMA issuer can start
         // the next tile.
         constexpr int kHalf = kSwapMaxTok / 2;  // token columns per thread and accumulator
-        SwapScheduler sched(group_lay, group_start, group_tiles_end, p.num_groups, num_w_blocks);
+        SwapScheduler sched(group_lay, group_start, group_tiles_end, p);
         SwapTile t;
         uint32_t iter = 0;
         const uint32_t q = warp & 3, half = (warp - 4) >> 2;
