@@ -692,6 +692,7 @@ struct MegaLayout {
 // per-tensor FP32 scales (device pointers; x_scale and act_scale hold one value and must be equal on every rank).
 struct LayerQuant {
     int kind = kKindFp8Fp4;
+    const float* logits = nullptr;     // [tokens, experts]: the layer routes first (into the buffer's topk_idx / topk_weights views)
     const float* x_scale = nullptr;    // scale of the NVFP4 input rows
     const float* act_scale = nullptr;  // calibrated scale the post-SwiGLU activations are quantised against
     const float* l1_scales = nullptr;  // [local experts] scales of the gate/up weights
@@ -1549,21 +1550,36 @@ int run_mega_moe(const LayerQuant& quant, void* y, const void* l1_w, const void*
     const float* topk_weights = reinterpret_cast<const float*>(base + l.topk_weights);
 
     struct ClearEvents { ~ClearEvents() { g_num_stage_events = 0; } } clear_events_on_exit;
+    // a small batch on one rank has its router inside the plan kernel
+    const bool small_plan = num_ranks == 1 && entries <= kPlanChunk && E <= 768;  // what fits 48 KB of shared memory
+    if (quant.logits != nullptr && num_tokens > 0) {
+        DGB_REQUIRE(num_experts <= 1024 && num_topk <= 32 && num_topk <= num_experts, "routing needs at most 1024 experts and topk in [1, min(32, experts)]");
+        if (!small_plan && (rc = dgb200_route_sigmoid_topk(quant.logits, num_tokens, num_experts, num_topk, reinterpret_cast<int64_t*>(base + l.topk_idx),
+                                                           reinterpret_cast<float*>(base + l.topk_weights), stream)))
+            return rc;
+    }
     if ((rc = record_stage(0, stream))) return rc;
     if (num_ranks > 1)
         return run_mega_moe_ep(quant, l, y, l1_w, l1_w_sf, l2_w, l2_w_sf, cumulative_local_expert_recv_stats, base, peer_buffer_ptrs, rank,
                                num_ranks, num_tokens, num_max_tokens_per_rank, num_experts, num_topk, hidden,
                                intermediate_hidden, activation_clamp, fast_math, stream);
 
-    // 1. dispatch plan: stable counting sort of the (token, k) entries by expert
-    DGB_CUDA(cudaMemsetAsync(src_of_row, 0xff, l.max_rows * 4, stream));
+    // 1. router (where the caller left it to the layer) and dispatch plan: stable counting sort of the (token, k) entries by expert
     const bool pdl = use_pdl();
-    DGB_CUDA(launch_kernel(dgb200_moe_count_kernel, dim3(chunks), dim3(kPlanChunk), E * sizeof(int), stream, pdl, topk_idx, entries, 0, E,
-                           chunk_hist));
-    DGB_CUDA(launch_kernel(dgb200_moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, chunk_hist, chunks, E, kSegmentAlignment,
-                           expert_start, expert_end, total_rows, cumulative_local_expert_recv_stats));
-    DGB_CUDA(launch_kernel(dgb200_moe_assign_kernel, dim3(chunks), dim3(kPlanChunk), 32 * E, stream, pdl, topk_idx, topk_weights, entries, 0,
-                           E, chunk_hist, expert_start, dest_row, src_of_row, row_weight));
+    if (small_plan) {
+        const size_t smem = kPlanChunk * 8 + 1024 * 8 + static_cast<size_t>(32) * E;
+        const auto plan = E <= 256 ? dgb200_moe_plan_small_kernel<8> : dgb200_moe_plan_small_kernel<32>;
+        DGB_CUDA(launch_kernel(plan, dim3(1), dim3(1024), smem, stream, pdl, quant.logits, const_cast<long long*>(topk_idx),
+                               const_cast<float*>(topk_weights), num_tokens, num_topk, E, kSegmentAlignment, expert_start, expert_end, total_rows,
+                               cumulative_local_expert_recv_stats, dest_row, src_of_row, row_weight));
+    } else {
+        DGB_CUDA(launch_kernel(dgb200_moe_count_kernel, dim3(chunks), dim3(kPlanChunk), E * sizeof(int), stream, pdl, topk_idx, entries, 0, E,
+                               chunk_hist));
+        DGB_CUDA(launch_kernel(dgb200_moe_scan_kernel, dim3(1), dim3(1024), 0, stream, pdl, chunk_hist, chunks, E, kSegmentAlignment,
+                               expert_start, expert_end, total_rows, cumulative_local_expert_recv_stats, src_of_row));
+        DGB_CUDA(launch_kernel(dgb200_moe_assign_kernel, dim3(chunks), dim3(kPlanChunk), 32 * E, stream, pdl, topk_idx, topk_weights, entries, 0,
+                               E, chunk_hist, expert_start, dest_row, src_of_row, row_weight));
+    }
 
     if ((rc = record_stage(1, stream))) return rc;
     // 2. gather quantised rows + scales into expert-sorted order
@@ -2244,17 +2260,8 @@ int dgb200_fp8_fp4_mega_moe_bf16_input(void* y, const void* x, int64_t x_row_str
                                        int32_t intermediate_hidden, float activation_clamp, int32_t fast_math, void* stream) {
     DGB_REQUIRE(x != nullptr && reinterpret_cast<uintptr_t>(x) % 16 == 0 && x_row_stride >= hidden && (x_row_stride * 2) % 16 == 0,
                 "x must be 16-byte aligned BF16 rows of at least `hidden` elements");
-    if (logits != nullptr && num_tokens > 0) {
-        MegaLayout l;
-        int rc = make_mega_layout(kKindFp8Fp4, num_ranks, num_experts, num_max_tokens_per_rank, num_topk, hidden, intermediate_hidden, &l);
-        if (rc) return rc;
-        DGB_REQUIRE(buffer != nullptr && num_tokens <= num_max_tokens_per_rank, "bad buffer or token count");
-        uint8_t* base = static_cast<uint8_t*>(buffer);
-        rc = dgb200_route_sigmoid_topk(logits, num_tokens, num_experts, num_topk, reinterpret_cast<int64_t*>(base + l.topk_idx),
-                                       reinterpret_cast<float*>(base + l.topk_weights), stream);
-        if (rc) return rc;
-    }
     LayerQuant quant;
+    quant.logits = logits;
     quant.x_bf16 = static_cast<const __nv_bfloat16*>(x);
     quant.x_bf16_row_stride = x_row_stride;
     return run_mega_moe(quant, y, l1_w, l1_w_sf, l2_w, l2_w_sf, cumulative_local_expert_recv_stats, buffer, peer_buffer_ptrs, rank,
@@ -2303,18 +2310,7 @@ int dgb200_fp8_fp4_mega_moe_ex(const dgb200_mega_moe_args* a, void* stream) {
         quant.peer_w[2] = a->peer_l2_w;
         quant.peer_w[3] = a->peer_l2_w_sf;
     }
-    if (a->logits != nullptr && a->num_tokens > 0) {
-        MegaLayout l;
-        int rc = make_mega_layout(kKindFp8Fp4, a->num_ranks, a->num_experts, a->num_max_tokens_per_rank, a->num_topk, a->hidden,
-                                  a->intermediate_hidden, &l, quant.shared_inter);
-        if (rc) return rc;
-        DGB_REQUIRE(a->buffer != nullptr && a->num_tokens <= a->num_max_tokens_per_rank, "bad buffer or token count");
-        uint8_t* base = static_cast<uint8_t*>(a->buffer);
-        rc = dgb200_route_sigmoid_topk(a->logits, a->num_tokens, a->num_experts, a->num_topk,
-                                       reinterpret_cast<int64_t*>(base + l.topk_idx), reinterpret_cast<float*>(base + l.topk_weights),
-                                       stream);
-        if (rc) return rc;
-    }
+    quant.logits = a->logits;
     return run_mega_moe(quant, a->y, a->l1_w, a->l1_w_sf, a->l2_w, a->l2_w_sf, a->cumulative_local_expert_recv_stats, a->buffer,
                         a->peer_buffer_ptrs, a->rank, a->num_ranks, a->num_tokens, a->num_max_tokens_per_rank, a->num_experts,
                         a->num_topk, a->hidden, a->intermediate_hidden, a->activation_clamp, a->fast_math,
@@ -2350,17 +2346,8 @@ int dgb200_nvfp4_mega_moe_bf16_input(void* y, const void* x, int64_t x_row_strid
                 "null per-tensor scale pointer");
     DGB_REQUIRE(x != nullptr && reinterpret_cast<uintptr_t>(x) % 16 == 0 && x_row_stride >= hidden && (x_row_stride * 2) % 16 == 0,
                 "x must be 16-byte aligned BF16 rows of at least `hidden` elements");
-    if (logits != nullptr && num_tokens > 0) {
-        MegaLayout l;
-        int rc = make_mega_layout(kKindNvfp4, 1, num_experts, num_max_tokens_per_rank, num_topk, hidden, intermediate_hidden, &l);
-        if (rc) return rc;
-        DGB_REQUIRE(buffer != nullptr && num_tokens <= num_max_tokens_per_rank, "bad buffer or token count");
-        uint8_t* base = static_cast<uint8_t*>(buffer);
-        rc = dgb200_route_sigmoid_topk(logits, num_tokens, num_experts, num_topk, reinterpret_cast<int64_t*>(base + l.topk_idx),
-                                       reinterpret_cast<float*>(base + l.topk_weights), stream);
-        if (rc) return rc;
-    }
     LayerQuant quant;
+    quant.logits = logits;
     quant.kind = kKindNvfp4;
     quant.x_scale = x_scale;
     quant.act_scale = act_scale;
@@ -2439,7 +2426,7 @@ int dgb200_moe_dispatch_plan_noalloc(const int64_t* topk_idx, int32_t num_tokens
     const long long* idx = reinterpret_cast<const long long*>(topk_idx);
     dgb200_moe_count_kernel<<<chunks, kPlanChunk, num_experts * sizeof(int), stream>>>(idx, n, 0, num_experts, chunk_hist);
     dgb200_moe_scan_kernel<<<1, 1024, 0, stream>>>(chunk_hist, chunks, num_experts, alignment, expert_start, expert_end,
-                                                    total_rows, nullptr);
+                                                    total_rows, nullptr, nullptr);
     if (n > 0)
         dgb200_ep_assign_kernel<<<chunks, kPlanChunk, 32 * num_experts, stream>>>(idx, n, num_experts, chunk_hist, expert_start,
                                                                               dest_row);

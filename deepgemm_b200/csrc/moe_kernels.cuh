@@ -40,13 +40,15 @@ dgb200_moe_count_kernel(const long long* __restrict__ topk_idx, int num_entries,
 }
 
 // One CTA. Turns chunk_hist into exclusive per-chunk bases, and produces per expert: count, aligned segment start,
-// segment end (the psum layout the grouped GEMM walks). total_rows[0] = end of the last segment.
+// segment end (the psum layout the grouped GEMM walks). total_rows[0] = end of the last segment. src_of_row (may be null): -1 into
+// every segment's padding rows; dgb200_moe_assign_kernel writes the others, and nothing reads past total_rows.
 __global__ void __launch_bounds__(1024)
 dgb200_moe_scan_kernel(int* __restrict__ chunk_hist, int num_chunks, int num_local_experts, int alignment,
                        int* __restrict__ expert_start, int* __restrict__ expert_end, int* __restrict__ total_rows,
-                       int* __restrict__ cumulative_stats) {
+                       int* __restrict__ cumulative_stats, int* __restrict__ src_of_row) {
     pdl_prologue();
     __shared__ int warp_sums[32];
+    __shared__ int pad_from[1024], pad_to[1024];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -54,11 +56,17 @@ dgb200_moe_scan_kernel(int* __restrict__ chunk_hist, int num_chunks, int num_loc
         const int e = base + static_cast<int>(threadIdx.x);
         int count = 0;
         if (e < num_local_experts) {
-            for (int c = 0; c < num_chunks; ++c) {
-                int* slot = chunk_hist + static_cast<long long>(c) * num_local_experts + e;
-                const int t = *slot;
-                *slot = count;
-                count += t;
+            // eight chunks' loads in flight (one after another, 128 chunks took 17 us)
+            int* slot = chunk_hist + e;
+            for (int c = 0; c < num_chunks; c += 8, slot += 8ll * num_local_experts) {
+                int t[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) t[i] = c + i < num_chunks ? slot[static_cast<long long>(i) * num_local_experts] : 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (c + i < num_chunks) slot[static_cast<long long>(i) * num_local_experts] = count;
+                    count += t[i];
+                }
             }
             if (cumulative_stats != nullptr) cumulative_stats[e] += count;
         }
@@ -86,8 +94,13 @@ dgb200_moe_scan_kernel(int* __restrict__ chunk_hist, int num_chunks, int num_loc
             expert_start[e] = start;
             expert_end[e] = start + count;
         }
+        pad_from[threadIdx.x] = start + count;
+        pad_to[threadIdx.x] = start + padded;
         __syncthreads();
         if (threadIdx.x == 1023) carry = start + padded;
+        if (src_of_row != nullptr)  // the padding rows of every segment have no source
+            for (int i = warp; i < min(1024, num_local_experts - base); i += 32)
+                for (int r = pad_from[i] + lane; r < pad_to[i]; r += 32) src_of_row[r] = -1;
         __syncthreads();
     }
     if (threadIdx.x == 0) total_rows[0] = carry;
@@ -127,6 +140,137 @@ dgb200_moe_assign_kernel(const long long* __restrict__ topk_idx, const float* __
     dest_row[i] = dest;
     src_of_row[dest] = i;
     row_weight[dest] = topk_weights[i];
+}
+
+// One token's route by one warp (expert e held by lane e % 32): lane k < topk receives the k-th largest logit's expert
+// (descending; ties -> lower expert index; 0x7fffffff where no logit above -infinity is left) and its sigmoid score
+// renormalised over the topk. Logits are compared as integers that order like the floats (0: taken, -infinity or NaN), so that one
+// reduction instruction finds the maximum and one the lowest expert that has it.
+template <int kMaxPerLane>
+__device__ __forceinline__ void route_token(const float* __restrict__ logits, int experts, int topk, int lane, int& my_idx, float& my_weight) {
+    uint32_t key[kMaxPerLane];
+#pragma unroll
+    for (int i = 0; i < kMaxPerLane; ++i) {
+        const int e = i * 32 + lane;
+        const float v = e < experts ? logits[e] : -INFINITY;
+        const uint32_t bits = __float_as_uint(v + 0.0f);  // -0 counts as +0
+        key[i] = v > -INFINITY ? (bits ^ ((bits >> 31) != 0 ? 0xffffffffu : 0x80000000u)) : 0u;
+    }
+    float my_best = -INFINITY;
+    my_idx = 0;
+    for (int k = 0; k < topk; ++k) {
+        uint32_t best = 0;
+#pragma unroll
+        for (int i = 0; i < kMaxPerLane; ++i) best = max(best, key[i]);
+        best = __reduce_max_sync(0xffffffffu, best);
+        uint32_t mine = 0x7fffffffu;
+#pragma unroll
+        for (int i = kMaxPerLane - 1; i >= 0; --i)
+            if (key[i] == best) mine = static_cast<uint32_t>(i * 32 + lane);
+        const uint32_t e = best == 0u ? 0x7fffffffu : __reduce_min_sync(0xffffffffu, mine);
+#pragma unroll
+        for (int i = 0; i < kMaxPerLane; ++i)
+            if (e == static_cast<uint32_t>(i * 32 + lane)) key[i] = 0u;
+        if (lane == k) {
+            my_idx = static_cast<int>(e);
+            my_best = best == 0u ? -INFINITY : __uint_as_float(best ^ ((best >> 31) != 0 ? 0x80000000u : 0xffffffffu));
+        }
+    }
+    const float my_score = 1.0f / (1.0f + expf(-my_best));
+    float sum = 0.0f;
+    for (int k = 0; k < topk; ++k) sum += __shfl_sync(0xffffffffu, my_score, k);
+    my_weight = my_score / sum;
+}
+
+// The whole dispatch plan of a small batch (at most kPlanChunk entries, 768 experts) in one CTA, the router before it included where
+// `logits` is given: what dgb200_route_sigmoid_topk_kernel and the count / scan / assign kernels write, in one launch instead of
+// four (4 tokens: 11 us of kernels, a memset and three more launches -> 6.8 us; the layer 155 -> 150).
+template <int kMaxPerLane>
+__global__ void __launch_bounds__(1024)
+dgb200_moe_plan_small_kernel(const float* __restrict__ logits, long long* __restrict__ topk_idx, float* __restrict__ topk_weights, int tokens,
+                             int topk, int experts, int alignment, int* __restrict__ expert_start, int* __restrict__ expert_end,
+                             int* __restrict__ total_rows, int* __restrict__ cumulative_stats, int* __restrict__ dest_row,
+                             int* __restrict__ src_of_row, float* __restrict__ row_weight) {
+    pdl_prologue();
+    extern __shared__ unsigned char plan_smem[];
+    int* entry_expert = reinterpret_cast<int*>(plan_smem);                   // [kPlanChunk]
+    float* entry_weight = reinterpret_cast<float*>(entry_expert + kPlanChunk);
+    int* start_of = reinterpret_cast<int*>(entry_weight + kPlanChunk);      // [1024]
+    int* end_of = start_of + 1024;
+    unsigned char* warp_hist = reinterpret_cast<unsigned char*>(end_of + 1024);  // [32 warps][experts], counts <= 32
+    __shared__ int warp_sums[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int entries = tokens * topk;
+    for (int i = threadIdx.x; i < 32 * experts; i += 1024) warp_hist[i] = 0;
+    if (logits != nullptr) {
+        for (int t = warp; t < tokens; t += 32) {
+            int idx;
+            float w;
+            route_token<kMaxPerLane>(logits + static_cast<long long>(t) * experts, experts, topk, lane, idx, w);
+            if (lane < topk) {
+                topk_idx[t * topk + lane] = idx;
+                topk_weights[t * topk + lane] = w;
+                entry_expert[t * topk + lane] = idx < experts ? idx : -1;
+                entry_weight[t * topk + lane] = w;
+            }
+        }
+    } else if (static_cast<int>(threadIdx.x) < entries) {
+        const long long g = topk_idx[threadIdx.x];
+        entry_expert[threadIdx.x] = g >= 0 && g < experts ? static_cast<int>(g) : -1;
+        entry_weight[threadIdx.x] = topk_weights[threadIdx.x];
+    }
+    __syncthreads();
+    // rank of each entry among the earlier ones of its expert: within the warp now, over the warps before it below
+    const int i = static_cast<int>(threadIdx.x);
+    const int e = i < entries ? entry_expert[i] : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, e);
+    const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
+    if (e >= 0 && rank_in_warp == 0) warp_hist[warp * experts + e] = static_cast<unsigned char>(__popc(peers));
+    __syncthreads();
+    int count = 0;
+    if (i < experts)
+        for (int w = 0; w < 32; ++w) count += warp_hist[w * experts + i];
+    const int padded = (count + alignment - 1) / alignment * alignment;
+    int incl = padded;
+    for (int off = 1; off < 32; off <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += n;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        int w = warp_sums[lane];
+        for (int off = 1; off < 32; off <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, w, off);
+            if (lane >= off) w += n;
+        }
+        warp_sums[lane] = w;
+    }
+    __syncthreads();
+    const int start = (warp > 0 ? warp_sums[warp - 1] : 0) + incl - padded;
+    if (i < experts) {
+        start_of[i] = start;
+        end_of[i] = start + count;
+        expert_start[i] = start;
+        expert_end[i] = start + count;
+        if (cumulative_stats != nullptr) cumulative_stats[i] += count;
+    }
+    if (i == 0) total_rows[0] = warp_sums[31];
+    __syncthreads();
+    for (int x = warp; x < experts; x += 32) {
+        const int end = end_of[x], to = (end + alignment - 1) / alignment * alignment;
+        for (int r = end + lane; r < to; r += 32) src_of_row[r] = -1;
+    }
+    if (i >= entries) return;
+    int dest = -1;
+    if (e >= 0) {
+        int before = 0;
+        for (int w = 0; w < warp; ++w) before += warp_hist[w * experts + e];
+        dest = start_of[e] + before + rank_in_warp;
+        src_of_row[dest] = i;
+        row_weight[dest] = entry_weight[i];
+    }
+    dest_row[i] = dest;
 }
 
 // Gathers quantised token rows and their packed scales into expert-sorted order. One CTA per 32 destination rows.
@@ -184,38 +328,12 @@ dgb200_route_sigmoid_topk_kernel(const float* __restrict__ logits, int tokens, i
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (t >= tokens) return;
-    float v[kMaxPerLane];
-#pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
-        const int e = i * 32 + lane;
-        v[i] = e < experts ? logits[static_cast<long long>(t) * experts + e] : -INFINITY;
-    }
-    float my_score = 0.0f, sum = 0.0f;
-    int my_idx = 0;
-    for (int k = 0; k < topk; ++k) {
-        float best = -INFINITY;
-        int best_e = 0x7fffffff;
-#pragma unroll
-        for (int i = 0; i < kMaxPerLane; ++i)
-            if (v[i] > best) { best = v[i]; best_e = i * 32 + lane; }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-            const int oe = __shfl_xor_sync(0xffffffffu, best_e, off);
-            if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-        }
-        if ((best_e & 31) == lane) {
-#pragma unroll
-            for (int i = 0; i < kMaxPerLane; ++i)
-                if (i == (best_e >> 5)) v[i] = -INFINITY;
-        }
-        const float score = 1.0f / (1.0f + expf(-best));
-        sum += score;
-        if (lane == k) { my_score = score; my_idx = best_e; }
-    }
+    int my_idx;
+    float my_weight;
+    route_token<kMaxPerLane>(logits + static_cast<long long>(t) * experts, experts, topk, lane, my_idx, my_weight);
     if (lane < topk) {
         topk_idx[static_cast<long long>(t) * topk + lane] = my_idx;
-        topk_weights[static_cast<long long>(t) * topk + lane] = my_score / sum;
+        topk_weights[static_cast<long long>(t) * topk + lane] = my_weight;
     }
 }
 
