@@ -473,14 +473,16 @@ struct SideStream {
     std::mutex mu;  // one fork .. join sequence at a time per device (the events are shared)
 };
 
-int side_stream_for_current_device(SideStream** out) {
+enum SideStreamUse { kSideGroupedSplit = 0, kSideSharedExperts = 1 };  // fork / join sequences that may nest have a stream each
+
+int side_stream_for_current_device(SideStreamUse use, SideStream** out) {
     constexpr int kMaxDevices = 64;
-    static SideStream table[kMaxDevices];
+    static SideStream table[2][kMaxDevices];
     static std::mutex create_mu;
     int dev = 0;
     DGB_CUDA(cudaGetDevice(&dev));
     DGB_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index %d out of range", dev);
-    SideStream& s = table[dev];
+    SideStream& s = table[use][dev];
     {
         std::lock_guard<std::mutex> lock(create_mu);
         if (s.stream == nullptr) {
@@ -959,7 +961,7 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
     // `first` on the caller's stream and `second` on the side stream, concurrently
     auto run_both = [&](GemmCall& first, auto&& second) -> int {
         SideStream* side = nullptr;
-        int rc1 = side_stream_for_current_device(&side);
+        int rc1 = side_stream_for_current_device(kSideGroupedSplit, &side);
         if (rc1) return rc1;
         std::lock_guard<std::mutex> lock(side->mu);
         DGB_CUDA(cudaEventRecord(side->fork, stream));
@@ -1609,14 +1611,30 @@ int run_mega_moe(const LayerQuant& quant, void* y, const void* l1_w, const void*
     }
 
     if ((rc = record_stage(2, stream))) return rc;
-    // 3 + 4. L1 (gate/up GEMM, fused SwiGLU + FP8 requant) and L2 (down GEMM, rows scattered to their combine slots)
-    rc = run_layer_gemms(quant, l, base, l1_w, l1_w_sf, l2_w, l2_w_sf, hidden, intermediate_hidden, activation_clamp, fast_math, stream, 3,
-                         static_cast<long long>(num_tokens) * num_topk / num_experts);
-    if (rc) return rc;
+    // 3 + 4. L1 (gate/up GEMM, fused SwiGLU + FP8 requant) and L2 (down GEMM)
+    auto routed_gemms = [&]() {
+        return run_layer_gemms(quant, l, base, l1_w, l1_w_sf, l2_w, l2_w_sf, hidden, intermediate_hidden, activation_clamp, fast_math, stream, 3,
+                               static_cast<long long>(num_tokens) * num_topk / num_experts);
+    };
     if (with_shared) {
-        if (quant.x_bf16 == nullptr && quant.kind != kKindBf16 && (rc = run_shared_x_sf(l, base, num_tokens, hidden, stream))) return rc;
-        if ((rc = run_shared_gemms(quant, l, base, num_tokens, hidden, activation_clamp, fast_math, stream))) return rc;
+        // The shared experts need nothing of the routed GEMMs: their two GEMMs run beside them, on the SMs that have no tile (a few
+        // tokens) or run out of tiles first. One after the other -> beside (64 experts): 1 token 121 -> 110 us, 128 tokens 354 -> 346,
+        // 4096 tokens 1696 -> 1643.
+        SideStream* side = nullptr;
+        if ((rc = side_stream_for_current_device(kSideSharedExperts, &side))) return rc;
+        std::lock_guard<std::mutex> lock(side->mu);
+        DGB_CUDA(cudaEventRecord(side->fork, stream));
+        DGB_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
+        rc = routed_gemms();
+        if (rc == 0 && quant.x_bf16 == nullptr && quant.kind != kKindBf16) rc = run_shared_x_sf(l, base, num_tokens, hidden, side->stream);
+        if (rc == 0) rc = run_shared_gemms(quant, l, base, num_tokens, hidden, activation_clamp, fast_math, side->stream);
+        // join even after a failed launch, so that the side stream never runs ahead of the caller's stream
+        DGB_CUDA(cudaEventRecord(side->join, side->stream));
+        DGB_CUDA(cudaStreamWaitEvent(stream, side->join, 0));
+    } else {
+        rc = routed_gemms();
     }
+    if (rc) return rc;
     // 5. combine: y[t] = sum over the top-k slots of the rows the L2 GEMM wrote
     PeerTable self{};
     self.p[0] = reinterpret_cast<unsigned long long>(base);
