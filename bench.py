@@ -930,12 +930,13 @@ def layer_line(args, cfg, rank, world, local_rank, steps, warmup, with_e2e=True,
 def kernels_of_one_step(nvfp4, world, local_experts, guests=0, comm_sms=0):
     """Launches of this library's kernels in one pass of the layer (memsets are not kernels of ours). FP8 layer on one
     rank: router, count, scan, assign, quantise + dispatch, the two GEMMs each split over the two tile orientations
-    (2 + 2 launches) plus the SwiGLU finisher, combine; NVFP4: router, count, scan, assign, quantise + dispatch, two GEMMs, combine. Expert parallel, P =
+    (2 + 2 launches) plus the SwiGLU finisher, combine; NVFP4: router, count, scan, assign, quantise + dispatch, the two GEMMs each as
+    whole pair tiles and remainders (2 + 2), combine. Expert parallel, P =
     phases (one with guest experts on one stream, else min(4, expert slots)): router, count, publish counts, flag, plan, assign, quantise, then per phase push + flag,
     flag + scale reorder + L1 + L2, return push + flag, and at the end a flag wait per phase and the combine; with guest
     experts one more launch fetches their weights and the guest slots count as experts."""
     if world == 1:
-        return 8 if nvfp4 else 11
+        return 10 if nvfp4 else 11
     phases = 1 if (guests and comm_sms <= 0) else min(4, local_experts + guests)
     return 7 + 9 * phases + 1 + (1 if guests else 0)
 
