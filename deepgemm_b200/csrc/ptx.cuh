@@ -202,6 +202,9 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* gmem_src, uint32_t 
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(gmem_src), "r"(bytes) : "memory");
 }
 
+// L2 prefetch of the line that holds one address.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
+
 // L2 prefetch of one box of a tiled tensor map (same coordinate rules as the load).
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t x, int32_t y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" :: "l"(map), "r"(x), "r"(y) : "memory");
