@@ -1182,7 +1182,7 @@ dgb200_moe_quant_dispatch_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long
         const uint32_t sf_byte = e4m3_byte(amax / 6.0f / s_t);
         const float factor = e4m3_to_float(sf_byte) * s_t;
         uint32_t lo, hi;
-        e2m1_codes_of_quotients(v, factor, special, lo, hi);
+        e2m1_codes_of_quotients(v, amax, factor, special, lo, hi);
         // packed scale int of 64 elements = the scale bytes of lanes L .. L + 3 (L a multiple of 4)
         const uint32_t b1 = __shfl_down_sync(0xffffffffu, sf_byte, 1), b2 = __shfl_down_sync(0xffffffffu, sf_byte, 2),
                        b3 = __shfl_down_sync(0xffffffffu, sf_byte, 3);

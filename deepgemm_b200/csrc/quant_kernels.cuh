@@ -81,14 +81,15 @@ __device__ __forceinline__ uint32_t e2m1x8_ladder(const float* v) {
 // The E2M1 codes of v[i] / factor (IEEE division) for 16 values, zero where factor is not positive. The quotient comes from the
 // correctly rounded reciprocal y by one residual step, q0 = v y, q = q0 + (v - q0 f) y (Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990), 3 operations instead of a division's; where the residual could
-// underflow, or v holds an infinity or NaN, the division itself is taken. The same bits as division and threshold ladder for
-// every BF16 mantissa and every FP32 mantissa of the factor. A division and seven compares per value bound the
-// stand-alone quantiser: 4096 x 7168 to NVFP4 55 -> 24 us; the ladder alone (to MXFP4) 45 -> 26.
-__device__ __forceinline__ void e2m1_codes_of_quotients(const float* v, float factor, bool special, uint32_t& lo, uint32_t& hi) {
+// underflow or the quotient overflow (`amax` = the largest |v|, a tensor scale far too small for the data), or v holds an infinity
+// or NaN, the division itself is taken. The same bits as division and threshold ladder for every BF16 mantissa and every FP32
+// mantissa of the factor. A division and seven compares per value bound the stand-alone quantiser: 4096 x 7168 to NVFP4
+// 55 -> 24 us; the ladder alone (to MXFP4) 45 -> 26.
+__device__ __forceinline__ void e2m1_codes_of_quotients(const float* v, float amax, float factor, bool special, uint32_t& lo, uint32_t& hi) {
     lo = hi = 0;
     if (!(factor > 0.0f)) return;
     float q[16];
-    if (special || !(factor > 0x1p-60f && factor < 0x1p60f)) {
+    if (special || !(factor > 0x1p-60f && factor < 0x1p60f) || amax > factor * 0x1p60f) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) q[i] = v[i] / factor;
         lo = e2m1x8_ladder(q);
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(256) dgb200_cast_rows_nvfp4_kernel(const CastN
         const uint32_t sf_byte = e4m3_byte(amax / 6.0f / s_t);
         const float factor = e4m3_to_float(sf_byte) * s_t;
         uint32_t lo, hi;
-        e2m1_codes_of_quotients(v, factor, special, lo, hi);
+        e2m1_codes_of_quotients(v, amax, factor, special, lo, hi);
         *reinterpret_cast<uint2*>(p.q + static_cast<long long>(row) * p.q_row_stride + col / 2) = make_uint2(lo, hi);
         sf_stage[warp * 4 + rr][lane] = static_cast<uint8_t>(sf_byte);
     }
