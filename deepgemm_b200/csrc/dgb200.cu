@@ -587,6 +587,7 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     DGB_REQUIRE(p.num_groups > 0 && p.num_groups <= kMaxCachedGroups, "at most %d groups", kMaxCachedGroups);
     DGB_REQUIRE(p.gran_a == 32 || (plain && p.gran_a == 128), "gran_k_a must be 32 (or 128), got %d", p.gran_a);
     DGB_REQUIRE(p.gran_b == 32 || (plain && p.gran_b == 128), "gran_k_b must be 32 (or 128), got %d", p.gran_b);
+    DGB_REQUIRE(c.a != nullptr && c.b != nullptr && c.sfa != nullptr && c.sfb != nullptr && p.layout != nullptr, "null tensor pointer");
     DGB_REQUIRE(reinterpret_cast<uintptr_t>(c.a) % 16 == 0 && reinterpret_cast<uintptr_t>(c.b) % 32 == 0 &&
                     reinterpret_cast<uintptr_t>(c.sfa) % 16 == 0 && reinterpret_cast<uintptr_t>(c.sfb) % 16 == 0,
                 "a and the scale factors must be 16-byte aligned, b 32-byte");

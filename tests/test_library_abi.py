@@ -85,6 +85,16 @@ def test_gemm_rejects_bad_arguments_before_touching_cuda(lib):
     assert rc == 1 and 'experts' in lib.dgb200_last_error().decode()
 
 
+@pytest.mark.parametrize('expected_m', [8, 64, 128, 256])
+@pytest.mark.parametrize('missing', ['a', 'sfa', 'b', 'sfb', 'masked_m'])
+def test_masked_gemm_rejects_null_tensors(lib, expected_m, missing):
+    """Whatever kernel the expected rows choose: the call ends before it asks the driver for anything."""
+    p = {name: ctypes.c_void_p(0 if name == missing else 4096) for name in ('a', 'sfa', 'b', 'sfb', 'masked_m')}
+    rc = lib.dgb200_m_grouped_fp8_fp4_gemm_nt_masked(p['a'], p['sfa'], 256, 256, p['b'], p['sfb'], 256, 256, ctypes.c_void_p(4096), 256,
+                                                     p['masked_m'], 2, 256, 256, 128, expected_m, 32, 32, 1, 0, ctypes.c_void_p(0))
+    assert rc == 1 and lib.dgb200_last_error().decode() == 'null tensor pointer'
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, '_lib', None)
     monkeypatch.setattr(_lib, 'LIB_PATH', str(tmp_path / 'libdgb200.so'))
