@@ -287,6 +287,8 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     p.sfa_group_rows = c.num_groups_a > 1 ? packed_k_a : 0;
     p.sfb_packed_k = packed_k_b;
     if (c.a_rows_total == 0) return 0;
+    DGB_REQUIRE((c.epilogue != kEpiBF16 && c.epilogue != kEpiF32) || reinterpret_cast<uintptr_t>(p.d) % 16 == 0,
+                "d must be 16-byte aligned");
 
     CUtensorMap tm_a, tm_b, tm_sfa, tm_sfb;
     int rc = 0;
@@ -601,6 +603,8 @@ int run_gemm_swap(GemmCall& c, cudaStream_t stream) {
     p.sfa_group_rows = c.num_groups_a > 1 ? packed_k_a : 0;
     p.sfb_packed_k = packed_k;
     if (c.a_rows_total == 0) return 0;
+    DGB_REQUIRE((c.epilogue != kEpiBF16 && c.epilogue != kEpiF32) || reinterpret_cast<uintptr_t>(p.d) % 16 == 0,
+                "d must be 16-byte aligned");
     CUtensorMap tm_x, tm_xs, tm_w, tm_sfx, tm_sfxs, tm_sfw;
     // Token slots of the small ring layout by the rows a group is expected to have: a group that exceeds them changes the
     // layout, which costs a drained ring, so the line lies where few groups do (10 rows expected: 1 in 40 has more than 16).

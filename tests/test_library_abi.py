@@ -95,6 +95,23 @@ def test_masked_gemm_rejects_null_tensors(lib, expected_m, missing):
     assert rc == 1 and lib.dgb200_last_error().decode() == 'null tensor pointer'
 
 
+@pytest.mark.parametrize('m', [8, 128, 4096])
+@pytest.mark.parametrize('d_is_fp32', [0, 1])
+@pytest.mark.parametrize('offset', [2, 4, 8])
+def test_gemms_reject_a_misaligned_output(lib, m, d_is_fp32, offset):
+    """All epilogues store 16 bytes at a time. Sizes on every route of the dense and the masked form: K split over a cluster,
+    whole tiles, tokens on either operand."""
+    p, d, null = ctypes.c_void_p(4096), ctypes.c_void_p(4096 + offset), ctypes.c_void_p(0)
+    message = 'd must be 16-byte aligned'
+    rc = lib.dgb200_bf16_gemm_nt(p, 8192, 0, p, 8192, 0, d, 512, m, 512, 8192, d_is_fp32, 0, null)
+    assert rc == 1 and lib.dgb200_last_error().decode() == message
+    rc = lib.dgb200_fp8_fp4_gemm_nt(p, p, m, p, p, 512, d, 512, m, 512, 8192, 32, 32, 1, d_is_fp32, 0, null)
+    assert rc == 1 and lib.dgb200_last_error().decode() == message
+    rc = lib.dgb200_m_grouped_fp8_fp4_gemm_nt_masked(p, p, m, 64 * m, p, p, 512, 64 * 512, d, 512, p, 2, m, 512, 8192, min(m, 1024),
+                                                     32, 32, 1, d_is_fp32, null)
+    assert rc == 1 and lib.dgb200_last_error().decode() == message
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, '_lib', None)
     monkeypatch.setattr(_lib, 'LIB_PATH', str(tmp_path / 'libdgb200.so'))
