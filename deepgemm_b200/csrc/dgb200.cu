@@ -185,18 +185,25 @@ bool use_pairs(const GemmCall& c, int block_n, int sms) {
     if (p.mode != kModeDense && p.mode != kModePsum && p.mode != kModeMasked) return false;
     if (p.rows_lo != 0 || p.rows_hi != 0 || p.ret_src != nullptr || p.push != nullptr) return false;
     if (p.row_part == kRowsTail) return false;
+    // Scale factors only in tcgen05.cp order (the layers; the public GEMMs take plain row order). The leader's tcgen05.cp reads both
+    // CTAs' copies, so a copy that a warp of the other CTA has turned must be released to it at cluster scope, which takes as long
+    // as the turned K blocks' MMAs: single CTAs -> pairs, dense FP8 4000 x 7168 x 2048 57 -> 63 us (scales per 128), FP8 x FP4 4096 x
+    // 7168 x 7168 170 -> 350 (per 32), NVFP4 8 groups of 1024 to 2048 rows, N 4096, K 7168 207 -> 430; with the leader
+    // writing both copies 57, 320 and 390.
+    if (c.kind != kKindBf16 && (p.sf_transposed == 0 || c.epilogue == kEpiF32)) return false;
     if (tuning().pair == 1 || p.row_part == kRowsPairs) return true;
     if (p.mode == kModeDense) {
-        // A pair tile takes about 0.87 of the time two single-CTA tiles take on the same two SMs (FP8 8192^3: 0.80, 4000 x
-        // 7168 x 2048: 0.85, BF16 4096 x 7168 x 2048: 0.90); with twice the granularity it may need another wave.
+        // A pair tile takes less time than two single-CTA tiles on the same two SMs (whole calls under sustained load, BF16: 4096 x
+        // 7168 x 2048 0.90 to 0.99, 8192^3 0.95 to 1.0); with twice the granularity it may need another wave, which nothing
+        // makes up for. 0.87 of a wave is where neither side of the line loses.
         const long long nb = p.n / 256;
         const long long single = (p.m + 127ll) / 128 * nb, pairs = (p.m + 255ll) / 256 * nb;
         const long long waves1 = (single + sms - 1) / sms, waves2 = (pairs + sms / 2 - 1) / (sms / 2);
         return p.m > 128 && waves2 * 87 < waves1 * 100;
     }
-    // Grouped: half a pair tile is lost on every second group. From 512 rows per group on that is less than what the pairs
-    // gain (8 groups of 1024 to 2048 rows, N 4096, K 7168: NVFP4 0.86 of the single-CTA time, BF16 0.95, FP8 x FP4 0.97). The
-    // psum layout only tells the rows the buffer holds, of which some are padding or free.
+    // Grouped (BF16, see above): half a pair tile is lost on every second group. From 512 rows per group on that is less than what
+    // the pairs gain (8 groups of 1024 to 2048 rows, N 4096, K 7168: 0.90 to 1.0 of the single-CTA time). The psum layout only
+    // tells the rows the buffer holds, of which some are padding or free.
     return c.expected_rows >= (p.mode == kModePsum ? 768 : 512);
 }
 
@@ -422,10 +429,8 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
                 if (bf16) return launch_gemm<256, kPairStages, kEpiBF16, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
                 if (nvfp4) return launch_gemm<256, kPairStagesNvfp4, kEpiBF16, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
                 return launch_gemm<256, kPairStages, kEpiBF16, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
-            case kEpiF32:
-                if (bf16) return launch_gemm<256, kPairStages, kEpiF32, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
-                if (nvfp4) return launch_gemm<256, kPairStagesNvfp4, kEpiF32, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
-                return launch_gemm<256, kPairStages, kEpiF32, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
+            case kEpiF32:  // (BF16 only: see use_pairs)
+                return launch_gemm<256, kPairStages, kEpiF32, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
             case kEpiSwiGLU: return launch_gemm<256, kPairStages, kEpiSwiGLU, kKindFp8Fp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
             case kEpiSwiGLUBf16: return launch_gemm<256, kPairStages, kEpiSwiGLUBf16, kKindBf16, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
             case kEpiSwiGLUNvfp4: return launch_gemm<256, kPairStagesNvfp4, kEpiSwiGLUNvfp4, kKindNvfp4, true>(tm_a, tm_b, tm_sfa, tm_sfb, tm_out, p, grid, stream);
@@ -2091,7 +2096,7 @@ int dgb200_per_channel_cast_to_fp8(const void* x, int32_t k, int32_t mn, int32_t
 int64_t dgb200_k_grouped_sf_workspace_bytes(int32_t num_groups, int32_t m, int32_t n, int32_t sum_k) {
     if (num_groups <= 0 || m <= 0 || n <= 0 || sum_k < 0) return 0;
     const long long rows = sum_k / 128 + 2ll * num_groups;  // one packed row per K block at most (scales per 32 K rows)
-    return rows * ((static_cast<long long>(m) + 3) / 4 * 4 + (static_cast<long long>(n) + 3) / 4 * 4) * 4;
+    return rows * ((static_cast<long long>(m) + 127) / 128 * 128 + (static_cast<long long>(n) + 127) / 128 * 128) * 4;
 }
 
 int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int32_t sf_rows, const void* b, const float* sfb,
@@ -2117,7 +2122,7 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
                     reinterpret_cast<uintptr_t>(sf_workspace) % 16 == 0,
                 "a, b and the workspace must be 16-byte aligned");
     const long long kp_rows = sum_k / 128 + 2ll * num_groups;
-    const long long aligned_m = (static_cast<long long>(m) + 3) / 4 * 4, aligned_n = (static_cast<long long>(n) + 3) / 4 * 4;
+    const long long aligned_m = (static_cast<long long>(m) + 127) / 128 * 128, aligned_n = (static_cast<long long>(n) + 127) / 128 * 128;
     uint32_t* sfa_packed = static_cast<uint32_t*>(sf_workspace);
     uint32_t* sfb_packed = sfa_packed + kp_rows * aligned_m;
     {
@@ -2141,6 +2146,7 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
     p.kg_psum = use_psum_layout ? 1 : 0;
     p.gran_a = p.gran_b = gran_k;
     p.b_fmt = kFmtE4M3;
+    p.sf_transposed = 1;  // dgb200_pack_k_grouped_sf_kernel writes tcgen05.cp order
     // Wide tiles halve the shared-memory fill per MMA cycle, which bounds the 128-wide tile (measured 1.1 - 1.8 vs
     // 1.7 - 2.0 PFLOP/s over 1024 .. 8192 K rows per group).
     const int block_n = tuning().block_n != 0 ? tuning().block_n : (n % 256 == 0 ? 256 : 128);

@@ -340,7 +340,7 @@ struct GemmSmem {
     static constexpr int kOffSfa = kOffB + kStages * kBBytes;
     static constexpr int kOffSfb = kOffSfa + kStages * kSfaBytes;
     static constexpr int kOffBar = kOffSfb + kStages * kSfbBytes;
-    static constexpr int kNumBars = (kPair ? 4 : 3) * kStages + 4;
+    static constexpr int kNumBars = 3 * kStages + 4;
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;
     static constexpr int kOffGroups = kOffMisc + 16;
     // Epilogue staging for TMA stores: 32 rows x 64 bytes per epilogue warp, in the 64-byte swizzle (512-byte atoms).
@@ -421,7 +421,6 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     uint64_t* sf_ready_bar = bars + 2 * kStages;
     uint64_t* tmem_full_bar = bars + 3 * kStages;
     uint64_t* tmem_empty_bar = bars + 3 * kStages + 2;
-    uint64_t* sf_full_bar = bars + 3 * kStages + 4;  // pairs only: this CTA's scale factors, see sf_local
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kOffMisc + 4);
 
@@ -430,17 +429,13 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
     const uint32_t cta_rank = kPair ? cluster_cta_rank() : 0u;
     const bool leader_cta = cta_rank == 0;
     const int tile_ctas = kPair ? 2 : (kSplitK ? static_cast<int>(cluster_num_ctas()) : 1);
-    // Pairs: scale factors in plain row order are transposed by a warp of the CTA they landed in, so they complete on a
-    // barrier of that CTA; everything else completes on the leader's barriers, where the MMA issuer waits.
-    const bool sf_local = kPair && kScaled && p.sf_transposed == 0;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int i = 0; i < kStages; ++i) {
             mbar_init(full_bar + i, 2 * kCtas);  // the A-side loader and the B-side loader of every CTA
             mbar_init(empty_bar + i, 1);         // tcgen05.commit of the MMA issuer
-            mbar_init(sf_ready_bar + i, sf_local ? 2 : 1);  // one lane of each transposer warp, after a warp barrier
-            if constexpr (kPair) mbar_init(sf_full_bar + i, 2);
+            mbar_init(sf_ready_bar + i, 1);      // one lane of the transposer warp, after a warp barrier
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(tmem_full_bar + i, 1);
@@ -537,19 +532,6 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         if constexpr (kPair) tma_load_2d_pair(smem + smem_off, map, map_to_cta(smem_u32(full_bar + stage), 0), x, y);
         else tma_load_2d(smem + smem_off, map, full_bar + stage, x, y);
     };
-    // a scale-factor load, or its absence in this K block
-    auto load_sf = [&](bool present, uint32_t bytes, int smem_off, const CUtensorMap* map, uint32_t stage, int x, int y) {
-        if (sf_local) {
-            if (present) {
-                mbar_arrive_expect_tx(sf_full_bar + stage, bytes);
-                tma_load_2d(smem + smem_off, map, sf_full_bar + stage, x, y);
-            } else {
-                mbar_arrive(sf_full_bar + stage);
-            }
-        } else if (present) {
-            load_tile(smem_off, map, stage, x, y);
-        }
-    };
 
     const int num_kb = p.k / kBlockK;
     // this CTA's K blocks, whole groups of 4 (what one packed scale int may cover); the host leaves no part empty
@@ -587,7 +569,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                     if (!ok) break;
                     const bool load_sfa = kScaled && kb % a_per == 0;
                     if (elect_one()) {
-                        stage_arrive(stage, L::kABytes + (load_sfa && !sf_local ? L::kSfaBytes : 0));
+                        stage_arrive(stage, L::kABytes + (load_sfa ? L::kSfaBytes : 0));
                         const int a_off = L::kOffA + stage * L::kABytes;
                         if constexpr (kKG) {
                             // MN-major A: one box per 128 bytes of M (128 E4M3 or 64 BF16 channels) x kBlockK K rows
@@ -601,8 +583,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                             for (int h = 0; h < 2; ++h) load_tile(a_off + h * 8192, &tm_a, stage, t.row_start + h * 64, kb * 64);
                         } else
                             load_tile(a_off, &tm_a, stage, kb * kTmaXPerKb, t.row_start);
-                        load_sf(load_sfa, L::kSfaBytes, L::kOffSfa + stage * L::kSfaBytes, &tm_sfa, stage, t.sf_row_start,
-                                sfa_y + kb * kSfInts / a_per);
+                        if (load_sfa) load_tile(L::kOffSfa + stage * L::kSfaBytes, &tm_sfa, stage, t.sf_row_start, sfa_y + kb * kSfInts / a_per);
                     }
                     __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -628,7 +609,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                     if (!ok) break;
                     const bool load_sfb = kScaled && kb % b_per == 0;
                     if (leader) {
-                        stage_arrive(stage, p.b_tx_bytes + (load_sfb && !sf_local ? L::kSfbBytes : 0));
+                        stage_arrive(stage, p.b_tx_bytes + (load_sfb ? L::kSfbBytes : 0));
                         const int b_off = L::kOffB + stage * L::kBBytes;
                         const int b_col = t.n_block * BLOCK_N + static_cast<int>(cta_rank) * kBRows;  // first channel of this CTA
                         if constexpr (kKG) {
@@ -650,8 +631,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                         } else
                             load_tile(b_off, &tm_b, stage, kb * kTmaXPerKb, t.group * p.n + b_col);
                         // the scales of all BLOCK_N channels: each CTA's tensor memory holds them
-                        load_sf(load_sfb, L::kSfbBytes, L::kOffSfb + stage * L::kSfbBytes, &tm_sfb, stage, t.n_block * BLOCK_N,
-                                sfb_y + kb * kSfInts / b_per);
+                        if (load_sfb) load_tile(L::kOffSfb + stage * L::kSfbBytes, &tm_sfb, stage, t.n_block * BLOCK_N, sfb_y + kb * kSfInts / b_per);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
@@ -701,12 +681,6 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                 ok = mbar_wait(((!kScaled || (p.sf_transposed && !kCpByHelper)) ? full_bar : sf_ready_bar) + stage, phase, abort_flag,
                                kTimeoutSfReady, kb);
                 if (!ok) break;
-                if constexpr (kPair && kScaled) {
-                    if (sf_local) {  // the transposers only waited for the scale factors
-                        ok = mbar_wait(full_bar + stage, phase, abort_flag, kTimeoutFull, kb);
-                        if (!ok) break;
-                    }
-                }
                 if (kCpByHelper && p.sf_transposed) tcgen05_fence_after();  // the helper warp's tcgen05.cp precede our MMAs
                 // No tcgen05 fence here: the data this wait covers was written to shared memory through the async proxy
                 // (TMA, or the transposer's stores followed by its proxy fence), not by tcgen05 operations.
@@ -785,12 +759,12 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
         Sched sched(p, group_layout, tile_ctas);
         Tile t;
         uint32_t stage = 0, phase = 0;
-        bool ok = kScaled && p.sf_transposed == 0;  // nothing to do when the scale factors arrive in tcgen05.cp order
+        bool ok = kScaled && !kPair && p.sf_transposed == 0;  // nothing to do when the scale factors arrive in tcgen05.cp order
         while (ok && sched.next(t)) {
             if (t.group < 0) continue;
             const int tile_kb = kKG ? t.num_kb : kb_hi;
             for (int kb = kb_lo; kb < tile_kb; ++kb) {
-                ok = mbar_wait((sf_local ? sf_full_bar : full_bar) + stage, phase, abort_flag, kTimeoutFull, kb);
+                ok = mbar_wait(full_bar + stage, phase, abort_flag, kTimeoutFull, kb);
                 if (!ok) break;
                 // All reads first, one warp barrier, then all writes: this warp serves every K block in turn, so its
                 // service time bounds the whole pipeline.
@@ -823,10 +797,7 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
-                    if (leader_cta) mbar_arrive(sf_ready_bar + stage);
-                    else mbar_arrive_cluster(map_to_cta(smem_u32(sf_ready_bar + stage), 0));
-                }
+                if (lane == 0) mbar_arrive(sf_ready_bar + stage);
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }

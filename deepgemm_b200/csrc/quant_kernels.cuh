@@ -366,8 +366,9 @@ dgb200_cast_channels_kernel(const __nv_bfloat16* __restrict__ x, int k, int mn, 
 // Scale factors of a K-grouped operand: FP32 powers of two [sum of ceil(k_g / gran_k) rows, mn], the groups' rows
 // concatenated (the reference's tests build them per group, tests/generators.py:413-435) -> packed UE8M0 ints, every
 // group starting on an int boundary: with gran_k = 128 int (j, col) of a group holds the exponent bytes of its K blocks
-// 4j .. 4j+3, with gran_k = 32 those of the four 32-row scales of K block j (zero past the group's end). One block row
-// per group (blockIdx.y); each block finds its group's first rows with a serial scan over the layout (at most a few
+// 4j .. 4j+3, with gran_k = 32 those of the four 32-row scales of K block j (zero past the group's end). Within every 128
+// columns the ints lie in tcgen05.cp order (sf_row_in_cp_order), so that the GEMM copies them without a
+// transposing pass; aligned_mn is a multiple of 128 and the columns past mn are zero. One block row per group (blockIdx.y); each block finds its group's first rows with a serial scan over the layout (at most a few
 // hundred groups). Reference: transform_k_grouped_sf_into_required_layout, csrc/apis/layout.hpp (called from
 // csrc/apis/gemm.hpp:335-336).
 __global__ void __launch_bounds__(256)
@@ -386,16 +387,16 @@ dgb200_pack_k_grouped_sf_kernel(const float* __restrict__ sf, int sf_rows, const
     }
     const int num_rows = (len + gran_k - 1) / gran_k;
     const int num_kp = (num_rows + 3) / 4;
-    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < static_cast<long long>(num_kp) * mn; i += gridDim.x * 256ll) {
-        const int j = static_cast<int>(i / mn), col = static_cast<int>(i - static_cast<long long>(j) * mn);
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < num_kp * aligned_mn; i += gridDim.x * 256ll) {
+        const int j = static_cast<int>(i / aligned_mn), col = static_cast<int>(i - j * aligned_mn);
         uint32_t packed = 0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int r = j * 4 + b;
-            if (r < num_rows && row0 + r < sf_rows)
+            if (col < mn && r < num_rows && row0 + r < sf_rows)
                 packed |= ((__float_as_uint(sf[static_cast<long long>(row0 + r) * mn + col]) >> 23) & 0xffu) << (8 * b);
         }
-        out[static_cast<long long>(kp0 + j) * aligned_mn + col] = packed;
+        out[static_cast<long long>(kp0 + j) * aligned_mn + sf_row_in_cp_order(col)] = packed;
     }
 }
 

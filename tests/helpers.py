@@ -1,9 +1,24 @@
 """Shared input builders for the parity tests: seeded CPU tensors quantised by the oracle."""
 import random
+import re
 
 import torch
 
 from oracle import quant
+
+
+def gemm_kernels_of(call):
+    """[(block_n, on pairs, K split)] of the tokens-on-M GEMM kernels that `call` launches, from the names the profiler sees."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    found = []
+    for event in prof.events():
+        name = re.sub(r'\((?:int|bool)\)', '', event.name)
+        match = re.search(r'dgb200_grouped_gemm_kernel<(\d+), \d+, \d+, \d+, (\w+), (\w+)>', name)
+        if match:
+            found.append((int(match[1]), match[2] in ('true', '1'), match[3] in ('true', '1')))
+    return found
 
 
 def quantize_groups(t: torch.Tensor, gran_k: int, fp4: bool):

@@ -1,5 +1,5 @@
-"""The GEMM kernel on CTA pairs (256 x 256 tiles) against the oracle at the sizes where its tiles can go wrong: rows around
-multiples of 128 and 256 (the second CTA of the last pair with no, one or all of its rows), groups that leave a remainder to
+"""The GEMM kernel on CTA pairs (256 x 256 tiles), and the forms that stay on single CTAs although pairs are asked for, against
+the oracle at the sizes where its tiles can go wrong: rows around multiples of 128 and 256 (the second CTA of the last pair with no, one or all of its rows), groups that leave a remainder to
 the single-CTA kernel, K around the depth of the operand ring, empty groups. Tolerances as for the single-CTA kernel:
 calc_diff <= 2e-3 (FP4 weights), <= 1e-3 (FP8 x FP8), < 1e-5 (BF16)."""
 import pytest
@@ -9,7 +9,7 @@ from oracle import gemm as ogemm
 from oracle import moe as omoe
 from oracle import nvfp4 as onv
 from oracle import quant
-from tests.helpers import moe_case, moe_case_nvfp4, quantize_groups
+from tests.helpers import gemm_kernels_of, moe_case, moe_case_nvfp4, quantize_groups
 
 pytestmark = pytest.mark.gpu
 
@@ -30,6 +30,42 @@ def _pairs_everywhere():
 
 
 ROWS = [(1, 256, 128), (127, 512, 768), (129, 256, 896), (256, 512, 1024), (257, 256, 128), (385, 512, 640), (700, 768, 2048)]
+
+
+@pytest.mark.parametrize('kind', ['fp8xfp8', 'fp8xfp4', 'nvfp4', 'masked', 'bf16', 'k_grouped_fp8', 'k_grouped_bf16'])
+def test_which_forms_run_on_pairs(dg, kind):
+    """Scale factors in plain row order stay on single CTAs, whatever the knob says: no CTA of a pair hands the other one shared
+    memory that its threads have written. The K-grouped form packs its scales in the order the tensor cores read."""
+    m, n, k = 512, 512, 512
+    ints = lambda rows, gran, groups=None: dg.transform_sf_into_required_layout(
+        torch.ones(*([groups] if groups else []), rows, k // gran, device='cuda'), rows, k, (1, gran), groups)
+    fp8 = lambda *shape: torch.ones(*shape, device='cuda').to(torch.float8_e4m3fn)
+    fp4 = lambda *shape: torch.zeros(*shape[:-1], shape[-1] // 2, dtype=torch.int8, device='cuda')
+    bf16 = lambda *shape: torch.ones(*shape, dtype=torch.bfloat16, device='cuda')
+    if kind in ('fp8xfp8', 'fp8xfp4'):
+        gran = 32 if kind == 'fp8xfp4' else 128
+        a, b = (fp8(m, k), ints(m, gran)), ((fp8 if kind == 'fp8xfp8' else fp4)(n, k), ints(n, gran))
+        call = lambda: dg.fp8_fp4_gemm_nt(a, b, bf16(m, n), recipe_a=(1, gran), recipe_b=(1, gran))
+    elif kind == 'nvfp4':
+        a = dg.per_token_cast_to_nvfp4(bf16(m, k))
+        sf = dg.pack_nvfp4_sf_mn_major(torch.ones(1, n, k // 16, device='cuda').to(torch.float8_e4m3fn))
+        layout = torch.tensor([m], dtype=torch.int32, device='cuda')
+        call = lambda: dg.m_grouped_nvfp4_gemm_nt_contiguous(a, (fp4(1, n, k), sf, torch.ones(1, device='cuda')), bf16(m, n), layout,
+                                                             use_psum_layout=True)
+    elif kind == 'masked':
+        counts = torch.tensor([m, m], dtype=torch.int32, device='cuda')
+        call = lambda: dg.m_grouped_fp8_fp4_gemm_nt_masked((fp8(2, m, k), ints(m, 128, 2)), (fp8(2, n, k), ints(n, 128, 2)), bf16(2, m, n),
+                                                           counts, m, recipe_a=(1, 128), recipe_b=(1, 128))
+    elif kind == 'bf16':
+        call = lambda: dg.bf16_gemm_nt(bf16(m, k), bf16(n, k), bf16(m, n))
+    else:
+        ks, d = torch.tensor([k], dtype=torch.int32, device='cuda'), torch.zeros(1, m, n, device='cuda')
+        if kind == 'k_grouped_fp8':
+            a, b = dg.utils.per_channel_cast_to_fp8(bf16(k, m), True), dg.utils.per_channel_cast_to_fp8(bf16(k, n), True)
+            call = lambda: dg.k_grouped_fp8_gemm_tn_contiguous(a, b, d, [k], ks, c=d)
+        else:
+            call = lambda: dg.k_grouped_bf16_gemm_tn_contiguous(bf16(k, m), bf16(k, n), d, [k], ks, c=d)
+    assert gemm_kernels_of(call) == [(256, kind in ('bf16', 'k_grouped_fp8', 'k_grouped_bf16'), False)]
 
 
 @pytest.mark.parametrize('m,n,k', ROWS)
