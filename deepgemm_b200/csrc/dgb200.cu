@@ -968,8 +968,14 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
     const bool pairs_and_tails = orient == kOrientM && (tuning().pair == 1 || (tuning().pair == -1 && expected_rows_per_expert >= pair_rows)) &&
                                  E <= kMaxCachedGroups && ret == nullptr && push == nullptr && (2 * intermediate_hidden) % 256 == 0 && hidden % 256 == 0 &&
                                  (tuning().block_n == 0 || tuning().block_n == 256);
-    // `first` on the caller's stream and `second` on the side stream, concurrently
+    bool limited = false;
+    if ((rc = sms_are_limited(&limited))) return rc;
+    // `first` on the caller's stream and `second` on the side stream, concurrently; one after the other under an SM limit
     auto run_both = [&](GemmCall& first, auto&& second) -> int {
+        if (limited) {
+            const int rc1 = run_gemm(first, stream);
+            return rc1 ? rc1 : second(stream);
+        }
         SideStream* side = nullptr;
         int rc1 = side_stream_for_current_device(kSideGroupedSplit, &side);
         if (rc1) return rc1;
@@ -1622,11 +1628,18 @@ int run_mega_moe(const LayerQuant& quant, void* y, const void* l1_w, const void*
 
     if ((rc = record_stage(2, stream))) return rc;
     // 3 + 4. L1 (gate/up GEMM, fused SwiGLU + FP8 requant) and L2 (down GEMM)
+    bool limited = false;
+    if ((rc = sms_are_limited(&limited))) return rc;
     auto routed_gemms = [&]() {
         return run_layer_gemms(quant, l, base, l1_w, l1_w_sf, l2_w, l2_w_sf, hidden, intermediate_hidden, activation_clamp, fast_math, stream, 3,
                                static_cast<long long>(num_tokens) * num_topk / num_experts);
     };
-    if (with_shared) {
+    auto shared_gemms = [&](cudaStream_t on) -> int {
+        int rc1 = 0;
+        if (quant.x_bf16 == nullptr && quant.kind != kKindBf16) rc1 = run_shared_x_sf(l, base, num_tokens, hidden, on);
+        return rc1 ? rc1 : run_shared_gemms(quant, l, base, num_tokens, hidden, activation_clamp, fast_math, on);
+    };
+    if (with_shared && !limited) {
         // The shared experts need nothing of the routed GEMMs: their two GEMMs run beside them, on the SMs that have no tile (a few
         // tokens) or run out of tiles first. One after the other -> beside (64 experts): 1 token 121 -> 110 us, 128 tokens 354 -> 346,
         // 4096 tokens 1696 -> 1643.
@@ -1636,13 +1649,13 @@ int run_mega_moe(const LayerQuant& quant, void* y, const void* l1_w, const void*
         DGB_CUDA(cudaEventRecord(side->fork, stream));
         DGB_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
         rc = routed_gemms();
-        if (rc == 0 && quant.x_bf16 == nullptr && quant.kind != kKindBf16) rc = run_shared_x_sf(l, base, num_tokens, hidden, side->stream);
-        if (rc == 0) rc = run_shared_gemms(quant, l, base, num_tokens, hidden, activation_clamp, fast_math, side->stream);
+        if (rc == 0) rc = shared_gemms(side->stream);
         // join even after a failed launch, so that the side stream never runs ahead of the caller's stream
         DGB_CUDA(cudaEventRecord(side->join, side->stream));
         DGB_CUDA(cudaStreamWaitEvent(stream, side->join, 0));
     } else {
         rc = routed_gemms();
+        if (rc == 0 && with_shared) rc = shared_gemms(stream);
     }
     if (rc) return rc;
     // 5. combine: y[t] = sum over the top-k slots of the rows the L2 GEMM wrote

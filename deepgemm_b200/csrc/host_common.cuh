@@ -65,6 +65,16 @@ inline int effective_num_sms(int* out) {
     return 0;
 }
 
+// The caller has limited the SMs, or some are reserved: kernels that would each fill what is left must not run side by side.
+inline int sms_are_limited(bool* out) {
+    int dev = 0, all = 0, usable = 0;
+    DGB_CUDA(cudaGetDevice(&dev));
+    DGB_CUDA(cudaDeviceGetAttribute(&all, cudaDevAttrMultiProcessorCount, dev));
+    if (const int rc = effective_num_sms(&usable)) return rc;
+    *out = usable < all;
+    return 0;
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -1,4 +1,5 @@
 """Shared input builders for the parity tests: seeded CPU tensors quantised by the oracle."""
+import json
 import random
 import re
 
@@ -19,6 +20,18 @@ def gemm_kernels_of(call):
         if match:
             found.append((int(match[1]), match[2] in ('true', '1'), match[3] in ('true', '1')))
     return found
+
+
+def kernel_launches(call, path):
+    """[(name, stream, CTAs, start, end)] of every kernel `call` launches, from a profiler trace written to `path`."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(path))
+    with open(path) as f:
+        events = [e for e in json.load(f)['traceEvents'] if e.get('cat') == 'kernel']
+    grid = lambda e: e['args']['grid'][0] * e['args']['grid'][1] * e['args']['grid'][2]
+    return [(e['name'], e['args']['stream'], grid(e), e['ts'], e['ts'] + e['dur']) for e in events]
 
 
 def quantize_groups(t: torch.Tensor, gran_k: int, fp4: bool):
