@@ -117,6 +117,60 @@ def test_masked(dg, kind):
     assert quant.calc_diff(got[mask], want[mask]) <= (1e-5 if kind == 'bf16' else 2e-3)
 
 
+@pytest.mark.parametrize('alignment', [16, 128])
+@pytest.mark.parametrize('zero_padding', [False, True])
+@pytest.mark.parametrize('mn_major', [False, True])
+def test_psum_bf16(dg, alignment, zero_padding, mn_major):
+    """Groups that start off the 128-row grid: the second CTA's rows may lie in the next group. Padding rows as asked."""
+    rows, n, k = [128, 0, 1, 129, 255, 256, 257, 385, 40], 512, 320
+    torch.manual_seed(alignment)
+    starts, ends, at = [], [], 0
+    for r in rows:
+        starts.append(at)
+        ends.append(at + r)
+        at += -(-r // alignment) * alignment
+    a = torch.zeros(at + 64, k).bfloat16()  # ... and rows no group owns at the end
+    for s, e in zip(starts, ends):
+        a[s:e] = torch.randn(e - s, k).bfloat16()
+    b, psum = (torch.randn(len(rows), n, k) * 0.05).bfloat16(), torch.tensor(ends, dtype=torch.int32)
+    want, mask = ogemm.bf16_grouped_gemm_contiguous(a, b, psum, use_psum_layout=True, alignment=alignment)
+    d = torch.full((a.size(0), n), float('nan'), dtype=torch.bfloat16, device='cuda')
+    b_in = b.cuda().transpose(1, 2).contiguous().transpose(1, 2) if mn_major else b.cuda()
+    before = dg.get_mk_alignment_for_contiguous_layout()
+    dg.set_mk_alignment_for_contiguous_layout(alignment)
+    try:
+        forms = gemm_kernels_of(lambda: dg.m_grouped_bf16_gemm_nt_contiguous(a.cuda(), b_in, d, psum.cuda(), use_psum_layout=True,
+                                                                             ensure_zero_padding=zero_padding))
+    finally:
+        dg.set_mk_alignment_for_contiguous_layout(before)
+    assert forms == [(256, True, False)]
+    got = d.cpu().float()
+    padding = torch.zeros_like(mask)
+    for s, e in zip(starts, ends):
+        padding[e:s + -(-(e - s) // alignment) * alignment] = True
+    assert quant.calc_diff(got[mask], want[mask]) < 1e-5
+    assert (got[padding] == 0).all() if zero_padding else torch.isnan(got[padding]).all()
+    assert torch.isnan(got[~mask & ~padding]).all()
+
+
+@pytest.mark.parametrize('rows,pairs', [([800, 801, 1023], True), ([300, 200, 500], False)])
+def test_psum_bf16_takes_pairs_by_itself(dg, rows, pairs):
+    from deepgemm_b200 import _lib
+    _lib.check(_lib.lib().dgb200_set_tuning(b'pair', -1))
+    n, k = 256, 256
+    torch.manual_seed(1)
+    ends, at = [], 0
+    for r in rows:
+        ends.append(at + r)
+        at += -(-r // 128) * 128
+    a, b, psum = torch.randn(at, k).bfloat16(), (torch.randn(3, n, k) * 0.05).bfloat16(), torch.tensor(ends, dtype=torch.int32)
+    want, mask = ogemm.bf16_grouped_gemm_contiguous(a, b, psum, use_psum_layout=True)
+    d = torch.zeros(at, n, dtype=torch.bfloat16, device='cuda')
+    forms = gemm_kernels_of(lambda: dg.m_grouped_bf16_gemm_nt_contiguous(a.cuda(), b.cuda(), d, psum.cuda(), use_psum_layout=True))
+    assert forms == [(256, pairs, False)]
+    assert quant.calc_diff(d.cpu()[mask], want[mask]) < 1e-5
+
+
 @pytest.mark.parametrize('m', [16, 144, 256, 272, 400])
 @pytest.mark.parametrize('kind', ['fp8', 'bf16'])
 @pytest.mark.parametrize('alias', [True, False])

@@ -1,5 +1,10 @@
 """The layer's GEMMs that run side by side on the library's own streams: which launches do, what an SM limit makes of them, CUDA
 graphs, and callers on several streams at once. The bits never depend on where a GEMM ran."""
+import os
+import subprocess
+import sys
+import threading
+
 import pytest
 import torch
 
@@ -8,6 +13,7 @@ from tests.helpers import kernel_launches, moe_case, quantize_groups
 
 pytestmark = pytest.mark.gpu
 HIDDEN, INTER, TOPK = 512, 256, 2
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.fixture(scope='module')
@@ -61,3 +67,75 @@ def test_an_sm_limit_holds(dg, tokens, experts, shared, tmp_path):
         dg.set_num_sms(0)
     assert len({k[1] for k in launches}) == 1 and max(k[2] for k in launches) <= limit
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize('tokens,experts,shared', CASES)
+def test_inside_a_cuda_graph(dg, tokens, experts, shared):
+    call, y = _layer(dg, tokens, experts, shared)
+    call()
+    torch.cuda.synchronize()
+    want = y.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for _ in range(2):
+        y.fill_(float('nan'))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+
+
+def test_first_call_of_a_process_inside_a_capture():
+    """The side streams and their events are made while the caller's stream is being captured."""
+    code = ('import torch, deepgemm_b200 as dg\n'
+            'from tests.test_side_streams_gpu import _layer\n'
+            'call, y = _layer(dg, 600, 4, True)\n'
+            'torch.cuda.synchronize()\n'
+            'graph = torch.cuda.CUDAGraph()\n'
+            'with torch.cuda.graph(graph):\n'
+            '    call()\n'
+            'graph.replay()\n'
+            'torch.cuda.synchronize()\n'
+            'replayed = y.clone()\n'
+            'y.fill_(float("nan"))\n'
+            'call()\n'
+            'torch.cuda.synchronize()\n'
+            'assert torch.equal(y, replayed) and not y.isnan().any()\n')
+    done = subprocess.run([sys.executable, '-c', code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_two_threads_on_two_streams(dg):
+    """Two callers share the side streams: their forks and joins must not mix. One layer of each kind of split."""
+    layers = [_layer(dg, 600, 4, True, seed=11), _layer(dg, 300, 4, True, seed=12)]
+    want = []
+    for call, y in layers:
+        call()
+        torch.cuda.synchronize()
+        want.append(y.clone())
+        y.fill_(float('nan'))
+    got, errors = [[], []], []
+
+    def work(i):
+        try:
+            call, y = layers[i]
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    call()
+                    got[i].append(y.clone())
+                    y.fill_(float('nan'))
+            stream.synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    for i in range(2):
+        assert len(got[i]) == 20 and all(torch.equal(y, want[i]) for y in got[i])
