@@ -1661,8 +1661,10 @@ int run_mega_moe(const LayerQuant& quant, void* y, const void* l1_w, const void*
     // 5. combine: y[t] = sum over the top-k slots of the rows the L2 GEMM wrote
     PeerTable self{};
     self.p[0] = reinterpret_cast<unsigned long long>(base);
+    int sms = 0;
+    if ((rc = effective_num_sms(&sms))) return rc;
     const int combine_passes = (hidden / 8 + 127) / 128;  // channels of a token in steps of one block
-    const int combine_columns = std::max(1, std::min(combine_passes, 148 * 8 / num_tokens));
+    const int combine_columns = std::max(1, std::min(combine_passes, sms * 8 / num_tokens));
     DGB_CUDA(launch_kernel(dgb200_moe_combine_kernel, dim3(num_tokens, combine_columns), dim3(128), (num_topk + 1) * sizeof(unsigned long long), stream, pdl,
                            self, l.l2_out, topk_idx, dest_row, num_topk, E, hidden,
                            with_shared ? reinterpret_cast<const __nv_bfloat16*>(base + l.shared_out) : nullptr,
