@@ -2066,7 +2066,10 @@ int dgb200_transform_sf_into_required_layout(const float* sf, int64_t stride_g, 
     p.psum_alignment = psum_alignment;
     const long long total = static_cast<long long>(num_groups) * ((sf_k + 3) / 4) * mn;
     const int grid = static_cast<int>(std::min<long long>((total + 255) / 256, 148 * 16));
-    DGB_CUDA(launch_kernel(dgb200_pack_sf_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), use_pdl(), p));
+    // Few scales launch ahead of their predecessor's end, many do not. Calls back to back, plain -> ahead (us): FP8 128 x 2048 x 7168 (7
+    // blocks here) 14.98 -> 14.78, 512 x 4096 x 4096 (16) 18.85 -> 18.70, 4000 x 7168 x 2048 (63) 55.7 -> 58.0.
+    const bool ahead = use_pdl() && grid <= 16;
+    DGB_CUDA(launch_kernel(dgb200_pack_sf_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), ahead, p));
     return 0;
 }
 

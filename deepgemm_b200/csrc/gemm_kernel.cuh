@@ -902,9 +902,11 @@ dgb200_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __gri
             };
             if constexpr (kKG) {
                 if (p.c != nullptr) {
-                    // Short K: the rest on its way into L2 while the tile's MMAs run, so that not every slab's load pays HBM latency (16
-                    // groups of 256 K rows, 2048 x 7168: 481 -> 396 us; 8 of 1024, 4096 x 4096: 308 -> 286). Where the MMAs of a tile
-                    // take longer than its slabs it gives nothing (8 of 4096 K rows, 2000 x 1024: 103 -> 105).
+                    // Short K: the rest on its way into L2 while the tile's MMAs run, so that not every slab's load pays HBM latency.
+                    // Measured in K blocks (128 FP8 or 64 BF16 rows, the same MMA time), never -> here -> always (us): FP8 16 groups of
+                    // 256 K rows, 2048 x 7168: 486 -> 385 -> 378; 8 of 1024, 4096 x 4096: 279 -> 254 -> 252; BF16 596 -> 525 and 302 ->
+                    // 297. Where a tile's MMAs take longer than its slabs it gives nothing or costs: FP8 8 of 4096, 4096 x 7168:
+                    // 914 -> 933 -> 979 and more, BF16 8 of 2048, 4096 x 4096: 424 -> 427 -> 434 and more.
                     if (t.num_kb <= 16 && (lane & 3) == 0) {
 #pragma unroll
                         for (int i = 1; i < kCols / 32; ++i)
