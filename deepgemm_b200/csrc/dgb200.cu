@@ -179,6 +179,25 @@ int mlp_kernel_choice() {
 // Pipeline stages of the pair kernels (the operand stages are 32 KB; NVFP4 adds 6 KB of scale factors to each, the others 1.5)
 constexpr int kPairStages = 6, kPairStagesNvfp4 = 5;
 
+int k_block_of(int kind) { return kind == kKindNvfp4 ? 256 : (kind == kKindBf16 ? 64 : 128); }
+
+// Does a GEMM of `tiles` 128 x 256 tiles with `k_blocks` K blocks each have the work that a pair kernel's later start (about 1.3 us)
+// costs? Single-CTA time -> pairs, BF16: one wave of tiles, 47 to 73 K blocks 1.04 to 1.07, 84 and more 0.87 to 0.94; two waves, 10 to
+// 24 blocks 1.01 to 1.05, 31 and more 0.90 to 0.97; three and more, 6 to 8 blocks 1.01 to 1.05, 9 and more 0.83 to 0.975.
+bool enough_for_pairs(long long tiles, long long k_blocks, int sms) {
+    const long long waves = (tiles + sms - 1) / sms;
+    return waves * k_blocks >= (waves <= 1 ? 80 : (waves == 2 ? 64 : 27));
+}
+
+// K blocks below which the pairs' epilogue (256 rows, one accumulator) costs more than their main loop saves, however many tiles
+// there are: gate/up of a layer with K 2048 (FP8) or 4096 (NVFP4) 1.05 to 1.3 of the single-CTA time, with K 4096 and 7168 less
+// than 1; the down GEMM with K 1024 and 1536 (NVFP4) 1.07 to 1.4, with K 2048 less than 1. BF16 has two accumulators.
+int min_pair_k_blocks(int kind, bool swiglu) {
+    if (kind == kKindBf16) return 1;
+    if (kind == kKindNvfp4) return swiglu ? 28 : 8;
+    return swiglu ? 32 : 16;
+}
+
 bool use_pairs(const GemmCall& c, int block_n, int sms) {
     const GemmParams& p = c.p;
     if (tuning().pair == 0 || block_n != 256 || sms < 2) return false;
@@ -192,19 +211,20 @@ bool use_pairs(const GemmCall& c, int block_n, int sms) {
     // writing both copies 57, 320 and 390.
     if (c.kind != kKindBf16 && (p.sf_transposed == 0 || c.epilogue == kEpiF32)) return false;
     if (tuning().pair == 1 || p.row_part == kRowsPairs) return true;
-    if (p.mode == kModeDense) {
-        // A pair tile takes less time than two single-CTA tiles on the same two SMs (whole calls under sustained load, BF16: 4096 x
-        // 7168 x 2048 0.90 to 0.99, 8192^3 0.95 to 1.0); with twice the granularity it may need another wave, which nothing
-        // makes up for. 0.87 of a wave is where neither side of the line loses.
-        const long long nb = p.n / 256;
-        const long long single = (p.m + 127ll) / 128 * nb, pairs = (p.m + 255ll) / 256 * nb;
-        const long long waves1 = (single + sms - 1) / sms, waves2 = (pairs + sms / 2 - 1) / (sms / 2);
-        return p.m > 128 && waves2 * 87 < waves1 * 100;
-    }
-    // Grouped (BF16, see above): half a pair tile is lost on every second group. From 512 rows per group on that is less than what
-    // the pairs gain (8 groups of 1024 to 2048 rows, N 4096, K 7168: 0.90 to 1.0 of the single-CTA time). The psum layout only
-    // tells the rows the buffer holds, of which some are padding or free.
-    return c.expected_rows >= (p.mode == kModePsum ? 768 : 512);
+    const bool swiglu = c.epilogue == kEpiSwiGLU || c.epilogue == kEpiSwiGLUBf16 || c.epilogue == kEpiSwiGLUNvfp4;
+    const int k_blocks = p.k / k_block_of(c.kind);
+    if (k_blocks < min_pair_k_blocks(c.kind, swiglu)) return false;
+    // Grouped: half a pair tile is lost on every second group. At 555 to 695 rows per group that is about what the pairs gain (BF16, 0.92
+    // to 1.06 of the single-CTA time), from 800 on it is less (0.89 to 0.98). The psum layout only tells the rows the buffer
+    // holds, of which some are padding or free.
+    const bool dense = p.mode == kModeDense;
+    const long long groups = dense ? 1 : p.num_groups, rows = dense ? p.m : c.expected_rows, nb = p.n / 256;
+    if (dense ? rows <= 128 : rows < 768) return false;
+    // A pair tile takes about 0.87 of the time of two single-CTA tiles on the same two SMs (see enough_for_pairs); with twice the
+    // granularity it may need another wave.
+    const long long single = groups * ((rows + 127) / 128) * nb, pairs = groups * ((rows + 255) / 256) * nb;
+    const long long waves1 = (single + sms - 1) / sms, waves2 = (pairs + sms / 2 - 1) / (sms / 2);
+    return waves2 * 87 < waves1 * 100 && enough_for_pairs(single, k_blocks, sms);
 }
 
 template <int BLOCK_N, int kStages>
@@ -256,7 +276,7 @@ int run_gemm(GemmCall& c, cudaStream_t stream) {
     GemmParams& p = c.p;
     const bool nvfp4 = c.kind == kKindNvfp4;
     const bool bf16 = c.kind == kKindBf16;
-    const int k_block = nvfp4 ? 256 : (bf16 ? 64 : 128);
+    const int k_block = k_block_of(c.kind);
     DGB_REQUIRE(p.k > 0 && p.k % k_block == 0, "k (%d) must be a positive multiple of %d", p.k, k_block);
     if (nvfp4 || bf16) p.gran_a = p.gran_b = 32;  // unused by these kinds; keeps the checks below uniform
     if (bf16) {
@@ -964,10 +984,23 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
     // pairs): FP8 x MXFP4, 64 experts: 256 rows each 1.00 -> 0.91 ms (0.95), 375 rows 1.33 -> 1.20 (1.28), 1024 rows 3.28 ->
     // 2.79 (2.83). NVFP4, 256 experts of 512 rows: 4.76 -> 4.29 ms (4.35); of 250 rows no difference. BF16: 512 rows 3.46 -> 3.24
     // (3.32); 375 rows 1.33 -> 1.37.
+    // The remainders are a second kernel that starts where the first one leaves SMs, one to two waves more in all, which a few
+    // experts do not pay for. One GEMM, single-CTA -> pairs and tails, by the waves of its pair tiles: BF16 below 3 1.2 to 1.6, from 3 to
+    // 10 0.87 to 1.07, above 0.84 to 1.05; FP8 gate/up 4 to 5 1.04 to 1.15, from 7 on 0.85 to 1.0, down 8 to 16 1.0 to 1.05, from 20 on 0.84
+    // to 0.98; NVFP4 gate/up 6 to 21 1.01 to 1.2, from 29 on 0.87 to 0.96, down 7 to 16 1.05 to 1.2, from 18 on 0.85 to 1.0.
     const long long pair_rows = nvfp4 ? 384 : (bf16 ? 448 : 192);
-    const bool pairs_and_tails = orient == kOrientM && (tuning().pair == 1 || (tuning().pair == -1 && expected_rows_per_expert >= pair_rows)) &&
-                                 E <= kMaxCachedGroups && ret == nullptr && push == nullptr && (2 * intermediate_hidden) % 256 == 0 && hidden % 256 == 0 &&
-                                 (tuning().block_n == 0 || tuning().block_n == 256);
+    int sms = 0;
+    if ((rc = effective_num_sms(&sms))) return rc;
+    auto pairs_and_tails = [&](const GemmCall& c) -> bool {
+        if (orient != kOrientM || tuning().pair == 0 || E > kMaxCachedGroups || ret != nullptr || push != nullptr) return false;
+        if ((2 * intermediate_hidden) % 256 != 0 || hidden % 256 != 0 || (tuning().block_n != 0 && tuning().block_n != 256)) return false;
+        if (tuning().pair == 1) return true;
+        const bool swiglu = c.epilogue != kEpiBF16;
+        const long long min_waves = bf16 ? 11 : (nvfp4 ? (swiglu ? 24 : 18) : (swiglu ? 7 : 20));
+        const long long pair_tiles = num_call_experts * expected_rows_per_expert / 256 * (c.p.n / 256);
+        return expected_rows_per_expert >= pair_rows && pair_tiles >= min_waves * std::max(sms / 2, 1) &&
+               c.p.k / k_block_of(c.kind) >= min_pair_k_blocks(c.kind, swiglu);
+    };
     bool limited = false;
     if ((rc = sms_are_limited(&limited))) return rc;
     // `first` on the caller's stream and `second` on the side stream, concurrently; one after the other under an SM limit
@@ -991,7 +1024,7 @@ int run_layer_gemms(const LayerQuant& quant, const MegaLayout& l, uint8_t* base,
     };
     auto run_split = [&](GemmCall& c) -> int {
         if (orient == kOrientSwapAll) return run_gemm_swap(c, stream);
-        if (orient == kOrientM && !pairs_and_tails) return run_gemm(c, stream);
+        if (orient == kOrientM && !pairs_and_tails(c)) return run_gemm(c, stream);
         GemmCall c2 = c;
         if (orient == kOrientM) {
             c.p.row_part = kRowsPairs;
@@ -2074,9 +2107,14 @@ int dgb200_transform_sf_into_required_layout(const float* sf, int64_t stride_g, 
 }
 
 namespace {
-bool use_pairs_k_grouped(int m, int block_n, int sms) {
+// Pairs where the problem is large enough, in waves of 128 x 256 tiles times K blocks of an average group (`k_blocks`: of all groups). Single-CTA time -> pairs:
+// below 28 1.02 to 1.33 (FP8 1 group of 512 K rows, 1552 x 2816 15.8 -> 21.1 us), 34 to 40 0.95 to 1.07, above 0.96 to 0.88, FP8 8 groups of 4096, 4096 x
+// 7168 0.92; with 2 to 8 K blocks and dozens of waves no difference.
+bool use_pairs_k_grouped(int num_groups, int m, int n, long long k_blocks, int block_n, int sms) {
     if (tuning().pair == 0 || block_n != 256 || sms < 2) return false;
-    return m > 128 || tuning().pair == 1;
+    if (tuning().pair == 1) return true;
+    const long long tiles = static_cast<long long>(num_groups) * ((m + 127) / 128) * (n / 256);
+    return m > 128 && (tiles + sms - 1) / sms * k_blocks >= 40ll * num_groups;
 }
 
 int k_grouped_grid(bool pair, int num_groups, int m, int n, int block_n, int sms) {
@@ -2172,7 +2210,7 @@ int dgb200_k_grouped_fp8_gemm_tn_contiguous(const void* a, const float* sfa, int
     int sms = 0;
     int rc = effective_num_sms(&sms);
     if (rc) return rc;
-    const bool pair = use_pairs_k_grouped(m, block_n, sms);
+    const bool pair = use_pairs_k_grouped(num_groups, m, n, sum_k / 128, block_n, sms);
     p.b_tx_bytes = (pair ? block_n / 2 : block_n) * 128;
     CUtensorMap tm_a, tm_b, tm_sfa, tm_sfb;
     rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),
@@ -2231,7 +2269,7 @@ int dgb200_k_grouped_bf16_gemm_tn_contiguous(const void* a, const void* b, const
     int sms = 0;
     int rc = effective_num_sms(&sms);
     if (rc) return rc;
-    const bool pair = use_pairs_k_grouped(m, block_n, sms);
+    const bool pair = use_pairs_k_grouped(num_groups, m, n, sum_k / 64, block_n, sms);
     p.b_tx_bytes = (pair ? block_n / 2 : block_n) * 128;
     CUtensorMap tm_a, tm_b;
     rc = make_tensor_map_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, static_cast<uint64_t>(m), static_cast<uint64_t>(sum_k),

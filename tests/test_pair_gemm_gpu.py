@@ -153,11 +153,12 @@ def test_psum_bf16(dg, alignment, zero_padding, mn_major):
     assert torch.isnan(got[~mask & ~padding]).all()
 
 
-@pytest.mark.parametrize('rows,pairs', [([800, 801, 1023], True), ([300, 200, 500], False)])
-def test_psum_bf16_takes_pairs_by_itself(dg, rows, pairs):
+@pytest.mark.parametrize('rows,k,pairs', [([800, 801, 1023], 5376, True), ([800, 801, 1023], 256, False), ([300, 200, 500], 5376, False)])
+def test_psum_bf16_takes_pairs_by_itself(dg, rows, k, pairs):
+    """Only with many rows per group and enough work in all."""
     from deepgemm_b200 import _lib
     _lib.check(_lib.lib().dgb200_set_tuning(b'pair', -1))
-    n, k = 256, 256
+    n = 512
     torch.manual_seed(1)
     ends, at = [], 0
     for r in rows:
@@ -169,6 +170,22 @@ def test_psum_bf16_takes_pairs_by_itself(dg, rows, pairs):
     forms = gemm_kernels_of(lambda: dg.m_grouped_bf16_gemm_nt_contiguous(a.cuda(), b.cuda(), d, psum.cuda(), use_psum_layout=True))
     assert forms == [(256, pairs, False)]
     assert quant.calc_diff(d.cpu()[mask], want[mask]) < 1e-5
+
+
+@pytest.mark.parametrize('m,n,k,pairs', [(4096, 4096, 1024, True), (1024, 512, 8192, True), (512, 512, 1024, False), (100, 4096, 8192, False)])
+def test_dense_and_k_grouped_take_pairs_by_themselves(dg, m, n, k, pairs):
+    from deepgemm_b200 import _lib
+    for name, value in ((b'pair', -1), (b'split_k', 0)):
+        _lib.check(_lib.lib().dgb200_set_tuning(name, value))
+    bf16 = lambda *shape: torch.ones(*shape, dtype=torch.bfloat16, device='cuda')
+    try:
+        assert gemm_kernels_of(lambda: dg.bf16_gemm_nt(bf16(m, k), bf16(n, k), bf16(m, n))) == [(256, pairs, False)]
+    finally:
+        _lib.check(_lib.lib().dgb200_set_tuning(b'split_k', -1))
+    m = -(-m // 8) * 8
+    ks, d = torch.tensor([k], dtype=torch.int32, device='cuda'), torch.zeros(1, m, n, device='cuda')
+    forms = gemm_kernels_of(lambda: dg.k_grouped_bf16_gemm_tn_contiguous(bf16(k, m), bf16(k, n), d, [k], ks, c=d))
+    assert forms == [(256, pairs, False)]
 
 
 @pytest.mark.parametrize('m', [16, 144, 256, 272, 400])

@@ -45,8 +45,17 @@ def _layer(dg, tokens, experts, shared, seed=7):
     return (lambda: dg.fp8_fp4_mega_moe(y, l1, l2, buf, **extra)), y
 
 
-# rows per expert: all GEMMs swapped; split by group size (about 150); whole pair tiles and remainders (about 300)
+# rows per expert: all GEMMs swapped; split by group size (about 150); whole pair tiles and remainders (about 300, so few experts only
+# with the knob)
 CASES = [(8, 8, True), (300, 4, False), (300, 4, True), (600, 4, False), (600, 4, True)]
+
+
+@pytest.fixture(autouse=True)
+def _pairs_and_remainders():
+    from deepgemm_b200 import _lib
+    _lib.check(_lib.lib().dgb200_set_tuning(b'pair', 1))
+    yield
+    _lib.check(_lib.lib().dgb200_set_tuning(b'pair', -1))
 
 
 @pytest.mark.parametrize('tokens,experts,shared', CASES)
@@ -88,7 +97,9 @@ def test_inside_a_cuda_graph(dg, tokens, experts, shared):
 def test_first_call_of_a_process_inside_a_capture():
     """The side streams and their events are made while the caller's stream is being captured."""
     code = ('import torch, deepgemm_b200 as dg\n'
+            'from deepgemm_b200 import _lib\n'
             'from tests.test_side_streams_gpu import _layer\n'
+            '_lib.check(_lib.lib().dgb200_set_tuning(b"pair", 1))\n'
             'call, y = _layer(dg, 600, 4, True)\n'
             'torch.cuda.synchronize()\n'
             'graph = torch.cuda.CUDAGraph()\n'
