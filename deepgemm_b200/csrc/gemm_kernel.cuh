@@ -374,6 +374,8 @@ constexpr int kRegsEpilogueWarps = 200; // ... to the two epilogue warpgroups, w
 // (nothing is multicast); both tensor cores read both halves. What bounds the single-CTA form with byte-wide (or BF16, or
 // NVFP4) weights is the operand bytes an SM takes from L2: 48 KB per K block, 96 bytes per cycle at full tensor rate against
 // about 60 it can get. A pair needs 32 KB per SM, and the smaller stages make the ring deeper (6 instead of 4 stages).
+// Scale factors come in tcgen05.cp order only, straight from TMA into each CTA: the leader's tcgen05.cp reads both CTAs' copies, and
+// what a thread of the other CTA had written there would have to be ordered before it at cluster scope (use_pairs).
 // kSplitK (dense mode): the CTAs of a cluster (2, 4 or 8) share ONE tile and take a part of its K each; every CTA leaves its FP32
 // accumulator in its own shared memory (the operand ring is done with) and then sums, rank by rank in a fixed order, one
 // slice of the tile's rows over the cluster. For problems with so few tiles that most SMs would idle while a few pull all of

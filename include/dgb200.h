@@ -32,8 +32,8 @@ extern "C" {
 const char* dgb200_last_error(void);
 int dgb200_version(void);
 
-/* Number of SMs persistent kernels are launched on (0 = all). Reference: set_num_sms / get_num_sms,
- * csrc/apis/runtime.hpp:12-20. */
+/* Number of SMs persistent kernels are launched on (0 = all). Below the device's number the layers run their GEMMs one after the
+ * other, so that the limit holds for all of them together. Reference: set_num_sms / get_num_sms, csrc/apis/runtime.hpp:12-20. */
 int dgb200_set_num_sms(int num_sms);
 int dgb200_get_num_sms(void);
 
@@ -45,6 +45,10 @@ int dgb200_get_num_sms(void);
  *                        rows per expert, tokens-on-M kernel otherwise), 0 = tokens-on-M kernel only, 1 = everything
  *                        through the swapped-operand kernel including its fused SwiGLU epilogue, 2 = the size split
  *                        with every expert of up to 160 rows on the swapped side (1 and 2: testing, experiments).
+ *   "split_k"            dense GEMMs: -1 (default) = K split over 2, 4 or 8 CTAs where few tiles have a long K, 0 = never (a row's
+ *                        bits then do not depend on the batch it is in), 2 / 4 / 8 = that split wherever the form exists.
+ *   "pair"               GEMMs on CTA pairs (256 x 256 tiles): -1 (default) = by size, 0 = never, 1 = wherever the form exists
+ *                        (BF16; FP8 and NVFP4 layers, whose scale factors lie in tcgen05.cp order; K-grouped). Same bits.
  *   "fused_dispatch"     expert-parallel layer with guest experts: 0 (default) = the dispatch push is a kernel of its own;
  *                        1 or a phase count 2..4 = several expert phases, and the epilogue warps of the gate/up GEMM of
  *                        phase q also push the rows this rank routes to phase q + 1 (measured slower than the default:
