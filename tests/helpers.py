@@ -1,37 +1,43 @@
 """Shared input builders for the parity tests: seeded CPU tensors quantised by the oracle."""
 import json
+import math
+import os
 import random
 import re
+import tempfile
 
+import pytest
 import torch
 
 from oracle import quant
 
 
+def kernel_launches(call, wanted='', repeats=3, attempts=6):
+    """[(name, stream, CTAs)] of the kernels with `wanted` in their names that `repeats` calls of `call` launch, from a profiler
+    trace. Now and then the profiler comes up too late for a short recording and sees none: then again; a machine where it sees
+    nothing at all skips the test."""
+    with tempfile.TemporaryDirectory() as folder:
+        path = os.path.join(folder, 'trace.json')
+        for _ in range(attempts):
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                for _ in range(repeats):
+                    call()
+                torch.cuda.synchronize()
+            prof.export_chrome_trace(path)
+            with open(path) as f:
+                events = [e for e in json.load(f)['traceEvents'] if e.get('cat') == 'kernel' and wanted in e['name']]
+            if events:
+                return [(re.sub(r'\((?:int|bool)\)', '', e['name']), e['args']['stream'], math.prod(e['args']['grid'])) for e in events]
+    pytest.skip('the profiler records no kernels here')
+
+
 def gemm_kernels_of(call):
-    """[(block_n, on pairs, K split)] of the tokens-on-M GEMM kernels that `call` launches, from the names the profiler sees."""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        call()
-        torch.cuda.synchronize()
-    found = []
-    for event in prof.events():
-        name = re.sub(r'\((?:int|bool)\)', '', event.name)
+    """{(block_n, on pairs, K split)} of the tokens-on-M GEMM kernels that `call` launches."""
+    found = set()
+    for name, _, _ in kernel_launches(call, 'dgb200_grouped_gemm_kernel'):
         match = re.search(r'dgb200_grouped_gemm_kernel<(\d+), \d+, \d+, \d+, (\w+), (\w+)>', name)
-        if match:
-            found.append((int(match[1]), match[2] in ('true', '1'), match[3] in ('true', '1')))
+        found.add((int(match[1]), match[2] in ('true', '1'), match[3] in ('true', '1')))
     return found
-
-
-def kernel_launches(call, path):
-    """[(name, stream, CTAs, start, end)] of every kernel `call` launches, from a profiler trace written to `path`."""
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        call()
-        torch.cuda.synchronize()
-    prof.export_chrome_trace(str(path))
-    with open(path) as f:
-        events = [e for e in json.load(f)['traceEvents'] if e.get('cat') == 'kernel']
-    grid = lambda e: e['args']['grid'][0] * e['args']['grid'][1] * e['args']['grid'][2]
-    return [(e['name'], e['args']['stream'], grid(e), e['ts'], e['ts'] + e['dur']) for e in events]
 
 
 def quantize_groups(t: torch.Tensor, gran_k: int, fp4: bool):

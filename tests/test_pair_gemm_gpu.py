@@ -65,7 +65,7 @@ def test_which_forms_run_on_pairs(dg, kind):
             call = lambda: dg.k_grouped_fp8_gemm_tn_contiguous(a, b, d, [k], ks, c=d)
         else:
             call = lambda: dg.k_grouped_bf16_gemm_tn_contiguous(bf16(k, m), bf16(k, n), d, [k], ks, c=d)
-    assert gemm_kernels_of(call) == [(256, kind in ('bf16', 'k_grouped_fp8', 'k_grouped_bf16'), False)]
+    assert gemm_kernels_of(call) == {(256, kind in ('bf16', 'k_grouped_fp8', 'k_grouped_bf16'), False)}
 
 
 @pytest.mark.parametrize('m,n,k', ROWS)
@@ -143,7 +143,7 @@ def test_psum_bf16(dg, alignment, zero_padding, mn_major):
                                                                              ensure_zero_padding=zero_padding))
     finally:
         dg.set_mk_alignment_for_contiguous_layout(before)
-    assert forms == [(256, True, False)]
+    assert forms == {(256, True, False)}
     got = d.cpu().float()
     padding = torch.zeros_like(mask)
     for s, e in zip(starts, ends):
@@ -168,7 +168,7 @@ def test_psum_bf16_takes_pairs_by_itself(dg, rows, k, pairs):
     want, mask = ogemm.bf16_grouped_gemm_contiguous(a, b, psum, use_psum_layout=True)
     d = torch.zeros(at, n, dtype=torch.bfloat16, device='cuda')
     forms = gemm_kernels_of(lambda: dg.m_grouped_bf16_gemm_nt_contiguous(a.cuda(), b.cuda(), d, psum.cuda(), use_psum_layout=True))
-    assert forms == [(256, pairs, False)]
+    assert forms == {(256, pairs, False)}
     assert quant.calc_diff(d.cpu()[mask], want[mask]) < 1e-5
 
 
@@ -179,13 +179,13 @@ def test_dense_and_k_grouped_take_pairs_by_themselves(dg, m, n, k, pairs):
         _lib.check(_lib.lib().dgb200_set_tuning(name, value))
     bf16 = lambda *shape: torch.ones(*shape, dtype=torch.bfloat16, device='cuda')
     try:
-        assert gemm_kernels_of(lambda: dg.bf16_gemm_nt(bf16(m, k), bf16(n, k), bf16(m, n))) == [(256, pairs, False)]
+        assert gemm_kernels_of(lambda: dg.bf16_gemm_nt(bf16(m, k), bf16(n, k), bf16(m, n))) == {(256, pairs, False)}
     finally:
         _lib.check(_lib.lib().dgb200_set_tuning(b'split_k', -1))
     m = -(-m // 8) * 8
     ks, d = torch.tensor([k], dtype=torch.int32, device='cuda'), torch.zeros(1, m, n, device='cuda')
     forms = gemm_kernels_of(lambda: dg.k_grouped_bf16_gemm_tn_contiguous(bf16(k, m), bf16(k, n), d, [k], ks, c=d))
-    assert forms == [(256, pairs, False)]
+    assert forms == {(256, pairs, False)}
 
 
 @pytest.mark.parametrize('m', [16, 144, 256, 272, 400])

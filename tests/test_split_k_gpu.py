@@ -45,10 +45,10 @@ def test_split_k(dg, split, m, n, k, block_n, kind):
         run = lambda d, c=None: dg.fp8_fp4_gemm_nt((a_q.cuda(), a_sf.cuda()), (b_q.cuda(), b_sf.cuda()), d, c, recipe_a=(1, gran_a),
                                                    recipe_b=(1, gran_b))
     d = torch.full((m, n), float('nan'), dtype=torch.bfloat16, device='cuda')
-    assert gemm_kernels_of(lambda: run(d)) == [(block_n, False, True)]
+    assert gemm_kernels_of(lambda: run(d)) == {(block_n, False, True)}
     assert quant.calc_diff(d.cpu(), want) <= tol
     f = torch.full((m, n), float('nan'), dtype=torch.float32, device='cuda')
-    assert gemm_kernels_of(lambda: run(f)) == [(block_n, False, True)]
+    assert gemm_kernels_of(lambda: run(f)) == {(block_n, False, True)}
     # FP32 partial sums of K products each: the relative error is far below the BF16 bound
     assert quant.calc_diff(f.cpu(), want) <= 1e-8
     c = torch.randn(m, n, device='cuda')
@@ -66,7 +66,7 @@ def test_the_rule_splits_by_itself(dg, m, n, k, form):
     """Without the knob: long K and few tiles split, short K does not."""
     a, b = torch.randn(m, k, device='cuda').bfloat16(), torch.randn(n, k, device='cuda').bfloat16()
     d = torch.empty(m, n, dtype=torch.bfloat16, device='cuda')
-    assert gemm_kernels_of(lambda: dg.bf16_gemm_nt(a, b, d)) == [form]
+    assert gemm_kernels_of(lambda: dg.bf16_gemm_nt(a, b, d)) == {form}
 
 
 def test_rows_do_not_depend_on_the_batch_without_the_split(dg):
